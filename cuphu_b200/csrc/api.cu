@@ -17,6 +17,7 @@
  *    never thrown across the ABI.
  */
 #include "kernels.cuh"
+#include "resident.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -346,11 +347,55 @@ struct JobOpts {
     double *wls_u = nullptr;
 };
 
+/* The solver of a job: the tiles of the plan that fit on the chip in one
+ * resident launch, the others in one streaming launch. */
+struct SolverJob {
+    ResidentPlan plan;
+    ResidentArgs res;                  /* device copies of the plan, and scratch */
+    std::vector<TileDesc> stream;      /* the streamed tiles, items renumbered */
+    const TileDesc *d_tiles = nullptr, *d_stream = nullptr;
+    const int *d_item = nullptr;
+    int stream_items = 0;
+    TileState *d_st = nullptr;
+    double *d_part = nullptr;
+    SolverCtl *d_ctl = nullptr;
+    int *d_pass = nullptr;
+    int pitch = 0, rows = 0, dev = 0, npass = 0;
+
+    int launch(bool fp64, const SolverPlanes &P, SolveParams sp, cudaStream_t s) const
+    {
+        sp.skip_block = solver_take_skip_block(dev);
+        sp.pass_iters = d_pass;
+        int rc = 0;
+        if (res.nblk) rc = launch_resident(res, d_tiles, P, d_ctl, sp, s);
+        if (!rc && !stream.empty())
+            rc = launch_solve(fp64, d_stream, d_item, stream_items, (int)stream.size(), P, pitch,
+                              rows, d_st, d_part, d_ctl, sp, dev, s);
+        return rc;
+    }
+    /* iteration statistics, after the launches are complete */
+    int stats(CuPhuSolveStats *st, int *err) const
+    {
+        SolverCtl ctl;
+        std::vector<int> pass(npass);
+        CUPHU_TRY_CUDA(cudaMemcpy(&ctl, d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+        CUPHU_TRY_CUDA(cudaMemcpy(pass.data(), d_pass, npass * sizeof(int), cudaMemcpyDeviceToHost));
+        st->total_iters = 0;
+        st->max_iters_pass = 0;
+        for (int n : pass) {
+            st->total_iters += n;
+            st->max_iters_pass = std::max(st->max_iters_pass, n);
+        }
+        st->px_iters = (double)ctl.px_iters;
+        *err = ctl.err;
+        return 0;
+    }
+};
+
 /* WLS mode of run_job: copy the caller's planes into the tile layout, one
  * solve without reweighting, raw FP64 solution out. */
 static int wls_job(const Plan &pl, SolverPlanes &P, const JobOpts &jo, cudaStream_t s,
-                   TileDesc *d_tiles, int *d_item, int ntiles, TileState *d_st, double *d_part,
-                   SolverCtl *d_ctl, float *d_deltas, int *d_pass, int dev, Workspace *W,
+                   const SolverJob &SJ, int ntiles, float *d_deltas, Workspace *W,
                    CuPhuSolveStats *stats)
 {
     const TileDesc &T = pl.tiles[0];
@@ -381,34 +426,30 @@ static int wls_job(const Plan &pl, SolverPlanes &P, const JobOpts &jo, cudaStrea
     sp.replace_every = jo.fp64 ? 0 : o.replace_every;
     sp.tol = o.tol;
     sp.deltas = d_deltas;
-    sp.pass_iters = d_pass;
     sp.timeout_ns = (long long)std::max(1, o.timeout_ms) * 1000000LL;
     sp.wls = 1;
     sp.warm = jo.wls_u0 ? 1 : 0;
     Timers tm(stats ? 2 : 0);
     cudaEvent_t e1 = tm.e[0], e2 = tm.e[1];
     if (stats) cudaEventRecord(e1, s);
-    int rc = launch_solve(jo.fp64, d_tiles, d_item, pl.nitems, ntiles, P, pl.pitch, pl.total_rows,
-                          d_st, d_part, d_ctl, sp, dev, s);
+    int rc = SJ.launch(jo.fp64, P, sp, s);
     if (rc) return rc;
     CUPHU_TRY_CUDA(cudaMemcpy2DAsync(jo.wls_u, (size_t)T.nc * 8, P.x, (size_t)T.pitch * 8,
                                      (size_t)T.nc * 8, T.nr, cudaMemcpyDeviceToDevice, s));
-    CUPHU_TRY_CUDA(cudaMemcpyAsync(W->status, &d_ctl->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUPHU_TRY_CUDA(cudaMemcpyAsync(W->status, &SJ.d_ctl->err, sizeof(int), cudaMemcpyDeviceToHost,
+                                   s));
     CUPHU_TRY_CUDA(cudaEventRecord(W->done, s));
     if (stats) {
         cudaEventRecord(e2, s);
         CUPHU_TRY_CUDA(cudaEventSynchronize(e2));
-        SolverCtl ctl;
-        CUPHU_TRY_CUDA(cudaMemcpy(&ctl, d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+        int err = 0;
+        if ((rc = SJ.stats(stats, &err))) return rc;
         float ms = 0;
         cudaEventElapsedTime(&ms, e1, e2);
         stats->ntiles = ntiles;
-        stats->total_iters = ctl.total_iters;
-        stats->max_iters_pass = ctl.max_pass_iters;
         stats->solve_ms = ms;
         stats->total_ms = ms;
-        stats->px_iters = (double)ctl.px_iters;
-        if (ctl.err) return fail(CUPHU_ERR_TIMEOUT, "solver grid barrier timed out");
+        if (err) return fail(CUPHU_ERR_TIMEOUT, "solver grid barrier timed out");
     }
     return 0;
 }
@@ -429,6 +470,20 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     const size_t vs = jo.fp64 ? sizeof(double) : sizeof(float);
     const size_t np = (size_t)pl.nplane;
 
+    /* which tiles the solver keeps on the chip; the rest are streamed, and
+     * only they need the planes of the PCG vectors */
+    SolverJob SJ;
+    int nsm = 0;
+    CUPHU_TRY_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    tune_note_items(0);
+    if (jo.fp64) {
+        for (int t = 0; t < ntiles; ++t) SJ.plan.streamed.push_back(t);
+    } else {
+        plan_resident(pl.tiles, nsm, SJ.plan);
+    }
+    const size_t nsched = SJ.plan.sched.size(), nstream = SJ.plan.streamed.size();
+    const size_t nps = nstream ? np : 0;
+
     /* device layout */
     size_t post_bytes = 0;
     for (auto &in : S)
@@ -448,8 +503,13 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
             cc_bytes = std::max(cc_bytes, (size_t)in.nrow * pitch * 12 + items * 4 +
                                               (size_t)in.nrow * 8 + 4096);
         }
-    TileDesc *d_cctd = nullptr;
-    char *d_ccbuf = nullptr;
+    TileDesc *d_cctd = nullptr, *d_stream = nullptr;
+    ResTile *d_sched = nullptr;
+    unsigned short *d_phys = nullptr;
+    int *d_boff = nullptr;
+    ResWork *d_work = nullptr;
+    unsigned *d_bars = nullptr;
+    char *d_ccbuf = nullptr, *d_rim = nullptr, *d_mail = nullptr;
     size_t need_phase = 0;
     for (auto &in : S)
         if (!in.ph_in) need_phase += (size_t)in.nrow * in.ncol;
@@ -464,15 +524,15 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
         P.wd = b.take<float>(np);
         P.wr = b.take<float>(np);
         P.x = b.take<double>(np);
-        P.dx = jo.fp64 ? nullptr : b.take<float>(np);
+        P.dx = jo.fp64 || !nstream ? nullptr : b.take<float>(np);
         P.bvec = jo.fp64 ? nullptr : b.take<double>(np);
-        P.r = b.take<char>(np * vs);
-        P.p0 = b.take<char>(np * vs);
-        P.p1 = b.take<char>(np * vs);
-        P.q = b.take<char>(np * vs);
-        P.diag = b.take<char>(np * vs);
+        P.r = b.take<char>(nps * vs);
+        P.p0 = b.take<char>(nps * vs);
+        P.p1 = b.take<char>(nps * vs);
+        P.q = b.take<char>(nps * vs);
+        P.diag = b.take<char>(jo.fp64 ? nps * vs : 0);
         P.z = b.take<char>(np * vs);
-        P.q1 = jo.fp64 ? nullptr : b.take<float>(np);
+        P.q1 = jo.fp64 ? nullptr : b.take<float>(nps);
         P.unw = b.take<float>(np);
         P.cyc = jo.want_cyc ? b.take<int32_t>(np) : nullptr;
         P.cont = jo.cont_out ? b.take<float>(np) : nullptr;
@@ -496,6 +556,11 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
         d_sout = b.take<SceneOut>(nsc);
         d_k = b.take<CostConsts>(nsc);
         d_cctd = b.take<TileDesc>(std::max(n_merge, 1));
+        d_stream = b.take<TileDesc>(std::max<size_t>(nstream, 1));
+        d_sched = b.take<ResTile>(std::max<size_t>(nsched, 1));
+        d_phys = b.take<unsigned short>(SJ.plan.phys.size() + 1);
+        d_boff = b.take<int>(SJ.plan.blk_off.size() + 1);
+        d_work = b.take<ResWork>(SJ.plan.work.size() + 1);
         d_st = b.take<TileState>(2 * (size_t)ntiles);
         /* item partials x2, published tile totals x2 (kNComp components
          * each), tile item tickets */
@@ -505,6 +570,9 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
         d_pass = b.take<int>(o.n_irls + 1);
         d_post = post_bytes ? b.take<char>(post_bytes) : nullptr;
         d_shift = b.take<SceneOut>(nsc);
+        d_bars = b.take<unsigned>(nsched);
+        d_rim = b.take<char>(resident_rim_bytes(SJ.plan.nblk));
+        d_mail = b.take<char>(resident_mail_bytes(SJ.plan.nblk));
         d_ccbuf = cc_bytes ? b.take<char>(cc_bytes) : nullptr;
     };
     SolverPlanes P = {};
@@ -593,6 +661,35 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
             cctd.push_back(T);
         }
     put(d_cctd, cctd.data(), cctd.size() * sizeof(TileDesc));
+    for (int t : SJ.plan.streamed) {
+        SJ.stream.push_back(pl.tiles[t]);
+        SJ.stream.back().item0 = SJ.stream_items;
+        SJ.stream_items += pl.tiles[t].nitems;
+    }
+    put(d_stream, SJ.stream.data(), nstream * sizeof(TileDesc));
+    put(d_sched, SJ.plan.sched.data(), nsched * sizeof(ResTile));
+    put(d_phys, SJ.plan.phys.data(), SJ.plan.phys.size() * sizeof(unsigned short));
+    put(d_boff, SJ.plan.blk_off.data(), SJ.plan.blk_off.size() * sizeof(int));
+    put(d_work, SJ.plan.work.data(), SJ.plan.work.size() * sizeof(ResWork));
+    SJ.res.sched = d_sched;
+    SJ.res.phys = d_phys;
+    SJ.res.blk_off = d_boff;
+    SJ.res.work = d_work;
+    SJ.res.rim = reinterpret_cast<unsigned long long *>(d_rim);
+    SJ.res.mail = reinterpret_cast<ulonglong2 *>(d_mail);
+    SJ.res.bars = d_bars;
+    SJ.res.nblk = SJ.plan.nblk;
+    SJ.d_tiles = d_tiles;
+    SJ.d_stream = d_stream;
+    SJ.d_item = d_item;
+    SJ.d_st = d_st;
+    SJ.d_part = d_part;
+    SJ.d_ctl = d_ctl;
+    SJ.d_pass = d_pass;
+    SJ.pitch = pl.pitch;
+    SJ.rows = pl.total_rows;
+    SJ.dev = dev;
+    SJ.npass = o.n_irls + 1;
 
     Timers tm(stats ? 4 : 0);
     cudaEvent_t e0 = tm.e[0], e1 = tm.e[1], e2 = tm.e[2], e3 = tm.e[3];
@@ -617,12 +714,15 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     }
     CUPHU_TRY_CUDA(cudaMemsetAsync(d_st, 0, 2 * ntiles * sizeof(TileState), s));
     CUPHU_TRY_CUDA(cudaMemsetAsync(d_ctl, 0, sizeof(SolverCtl), s));
-    CUPHU_TRY_CUDA(cudaMemsetAsync(d_part + 2 * (size_t)kNComp * pl.nitems +
-                                       2 * (size_t)kNComp * ntiles,
-                                   0, (size_t)ntiles * sizeof(double), s));
+    CUPHU_TRY_CUDA(cudaMemsetAsync(d_pass, 0, (o.n_irls + 1) * sizeof(int), s));
+    if (nsched) CUPHU_TRY_CUDA(cudaMemsetAsync(d_bars, 0, nsched * sizeof(unsigned), s));
+    /* the streaming solver's tile tickets follow its partials and totals */
+    if (nstream)
+        CUPHU_TRY_CUDA(cudaMemsetAsync(d_part + 2 * (size_t)kNComp * SJ.stream_items +
+                                           2 * (size_t)kNComp * nstream,
+                                       0, nstream * sizeof(double), s));
 
-    if (jo.wls) return wls_job(pl, P, jo, s, d_tiles, d_item, ntiles, d_st, d_part, d_ctl,
-                               d_deltas, d_pass, dev, W, stats);
+    if (jo.wls) return wls_job(pl, P, jo, s, SJ, ntiles, d_deltas, W, stats);
     for (int i = 0; i < nsc; ++i) {
         if (S[i].ph_in) continue;
         long long n = (long long)S[i].nrow * S[i].ncol;
@@ -643,11 +743,9 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     sp.replace_every = jo.fp64 ? 0 : o.replace_every;
     sp.tol = o.tol;
     sp.deltas = d_deltas;
-    sp.pass_iters = d_pass;
     sp.timeout_ns = (long long)std::max(1, o.timeout_ms) * 1000000LL;
     if (stats) cudaEventRecord(e1, s);
-    rc = launch_solve(jo.fp64, d_tiles, d_item, pl.nitems, ntiles, P, pl.pitch, pl.total_rows, d_st,
-                      d_part, d_ctl, sp, dev, s);
+    rc = SJ.launch(jo.fp64, P, sp, s);
     if (rc) return rc;
     if (stats) cudaEventRecord(e2, s);
     if (jo.want_cc) {
@@ -731,18 +829,15 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     if (stats) {
         cudaEventRecord(e3, s);
         CUPHU_TRY_CUDA(cudaEventSynchronize(e3));
-        SolverCtl ctl;
-        CUPHU_TRY_CUDA(cudaMemcpy(&ctl, d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+        int err = 0;
+        if ((rc = SJ.stats(stats, &err))) return rc;
         float ms_solve = 0, ms_total = 0;
         cudaEventElapsedTime(&ms_solve, e1, e2);
         cudaEventElapsedTime(&ms_total, e0, e3);
         stats->ntiles = ntiles;
-        stats->total_iters = ctl.total_iters;
-        stats->max_iters_pass = ctl.max_pass_iters;
         stats->solve_ms = ms_solve;
         stats->total_ms = ms_total;
-        stats->px_iters = (double)ctl.px_iters;
-        if (ctl.err) return fail(CUPHU_ERR_TIMEOUT, "solver grid barrier timed out");
+        if (err) return fail(CUPHU_ERR_TIMEOUT, "solver grid barrier timed out");
     }
     return cuda_fail(cudaGetLastError(), "unwrap pipeline");
 }

@@ -69,8 +69,8 @@ struct TileState {
 struct SolverCtl {
     unsigned bar_count, bar_gen;
     int err, n_active, snap;
-    int total_iters, max_pass_iters;
     int pass_max;                  /* largest iteration count of the current pass (mixed) */
+    unsigned progress;             /* grows while resident tiles iterate */
     unsigned long long px_iters;   /* sum over tiles and passes of iterations x pixels */
 };
 
@@ -78,7 +78,8 @@ struct SolveParams {
     int n_irls, max_iter, replace_every;
     float tol;
     const float *deltas;        /* per-pass IRLS delta (host powf schedule) */
-    int *pass_iters;            /* [n_irls+1] iterations per pass (out)     */
+    int *pass_iters;            /* [n_irls+1] largest iteration count of a tile
+                                   per pass (in: 0, out)                     */
     long long timeout_ns;       /* grid-barrier wait limit                   */
     int wls = 0;                /* raw solve: no anchor / congruence phase   */
     int warm = 0;               /* keep the caller's initial x on pass 0     */
@@ -88,6 +89,8 @@ struct SolveParams {
 
 /* laplace.cu: arm the failure test for the next solver launch on a device */
 void solver_skip_barrier_once(int dev, int block);
+/* the armed block (-1: none); disarms */
+int solver_take_skip_block(int dev);
 
 struct ScenePlan {
     float *unw_out;

@@ -1,0 +1,91 @@
+"""The on-chip solver (mixed precision, tiles that fit the chip) at the sizes
+where its split can go wrong: single rows and columns, items exactly filled
+and one pixel over, groups with idle members, ragged last levels, the largest
+tile it takes and the first one it leaves to the streaming solver.  The
+reference is the FP64 streaming solve of the same tile, which the other tests
+pin to the oracle bit for bit.  The bounds are those of the mixed mode
+elsewhere: 1e-3 rad RMS of the continuous solution and 1e-4 of the cycles,
+with the floor of 3 that a handful of half-cycle pixels needs."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from cuphu_b200 import synthetic as S
+from cuphu_b200._lib import (CuPhuScene, CuPhuSolveStats, check, default_params,
+                             default_solve_options, lib)
+from tests.devbuf import dptr, empty, to_dev, to_host
+from tests.test_gpu_laplace import gpu_solve
+
+pytestmark = pytest.mark.gpu
+
+
+def scene(nr, nc, seed, blocked=False):
+    """(costs, phase): arc variances from a smooth coherence, and with
+    ``blocked`` a band of arcs that carry no weight."""
+    ig, g, _, _ = S.bumps(nr, nc, seed=seed, nbumps=3, amp_range=(5.0, 25.0),
+                          sigma_range=(8.0, 60.0))
+    ph = np.mod(np.angle(ig), 2 * np.pi).astype(np.float32)
+    rng = np.random.default_rng(seed)
+    narcs = (nr - 1) * nc + nr * (nc - 1)
+    costs = np.zeros((max(narcs, 1), 2), np.int16)
+    nra = (nr - 1) * nc
+    costs[:nra, 1] = (1 + 80 * (1 - g[:-1].reshape(-1))).astype(np.int16)
+    costs[nra:narcs, 1] = (1 + 80 * (1 - g[:, 1:].reshape(-1))).astype(np.int16)
+    if blocked and narcs > 40:
+        a = int(rng.integers(0, narcs // 2))
+        costs[a:a + narcs // 7, 1] = 32000
+    return costs, ph
+
+
+@pytest.mark.parametrize("shape,blocked", [
+    ((1, 1), False), ((1, 70), False), ((70, 1), False), ((2, 64), False), ((16, 64), True),
+    ((17, 65), False), ((15, 1037), True), ((1025, 63), False), ((255, 1030), False),
+    ((512, 512), True), ((967, 961), False), ((1000, 1102), True), ((1344, 1340), False),
+    ((1424, 1409), False)])
+def test_on_chip_solve_matches_fp64(torch_cuda, shape, blocked):
+    costs, ph = scene(*shape, seed=shape[0] + 3 * shape[1], blocked=blocked)
+    _, k64, c64, s64 = gpu_solve(torch_cuda, costs, ph, precision=1, n_irls=2)
+    _, k32, c32, s32 = gpu_solve(torch_cuda, costs, ph, precision=0, n_irls=2)
+    rms = float(np.sqrt(np.mean((c32.astype(np.float64) - c64) ** 2)))
+    assert rms < 1e-3, rms
+    assert int(np.sum(k32 != k64)) <= max(3, int(1e-4 * k64.size))
+    assert abs(s32.total_iters - s64.total_iters) <= 3 + s64.total_iters // 50
+
+
+def test_batch_of_on_chip_and_streamed_tiles(torch_cuda):
+    """One job whose tiles go both ways, some sharing the chip side by side:
+    every scene's outputs equal those of its own call."""
+    shapes = [(60, 50), (1500, 1530), (300, 340), (1, 90), (512, 512)]
+    p = default_params()
+    o = default_solve_options(precision=0, n_irls=1, max_iter=120)
+    data = []
+    for i, sh in enumerate(shapes):
+        ig, g, _, _ = S.bumps(*sh, seed=70 + i, nbumps=2, amp_range=(5, 20), sigma_range=(8, 20))
+        ph = np.mod(np.angle(ig), 2 * np.pi).astype(np.float32)
+        data.append((to_dev(ph), to_dev(g)))
+
+    def call(which):
+        scenes = (CuPhuScene * len(which))()
+        out = []
+        for j, i in enumerate(which):
+            du = empty(shapes[i], torch_cuda.float32)
+            dc = empty(shapes[i], torch_cuda.int32)
+            out.append((du, dc))
+            scenes[j] = CuPhuScene(None, data[i][0].data_ptr(), data[i][1].data_ptr(), None, None,
+                                   shapes[i][0], shapes[i][1], 1, 1, 0, 0, 5.0, du.data_ptr(),
+                                   dc.data_ptr())
+        st = CuPhuSolveStats()
+        check(lib().cuphu_unwrap_batch_device(scenes, len(which), 0, C.byref(p), C.byref(o),
+                                              C.byref(st), None))
+        return [(to_host(u), to_host(c)) for u, c in out], st
+
+    got, st = call(range(len(shapes)))
+    assert st.ntiles == len(shapes)
+    longest = 0
+    for i in range(len(shapes)):
+        want, one = call([i])
+        longest = max(longest, one.max_iters_pass)
+        assert np.array_equal(got[i][0].view(np.int32), want[0][0].view(np.int32))
+        assert np.array_equal(got[i][1], want[0][1])
+    assert st.max_iters_pass == longest
