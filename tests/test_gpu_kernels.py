@@ -157,6 +157,24 @@ def test_residues_match_oracle_and_conserve(torch_cuda):
     assert (res != 0).sum() > 0
 
 
+@pytest.mark.parametrize("shape", [(2, 2), (2, 33), (9, 32), (10, 31), (17, 250), (8, 249), (300, 2)])
+def test_residues_at_strip_edges(torch_cuda, shape):
+    """Strips of 31 columns and 8 rows: exactly filled, one over, one short;
+    phases outside [0, 2 pi) and NaN included."""
+    rng = np.random.default_rng(shape[0] * 1000 + shape[1])
+    ph = rng.uniform(0, 2 * np.pi, shape).astype(np.float32)
+    ph[0, 0] = -7.5
+    ph[-1, -1] = 40.0
+    ph[shape[0] // 2, shape[1] // 2] = np.nan
+    dr = empty((shape[0] - 1, shape[1] - 1), torch_cuda.int8)
+    check(lib().cuphu_residues_gpu(dptr(to_dev(ph)), shape[0], shape[1], dptr(dr), None))
+    got, want = to_host(dr), O.residues(ph)
+    # a residue with a NaN corner has no defined value
+    bad = np.isnan(ph)
+    touched = bad[:-1, :-1] | bad[1:, :-1] | bad[:-1, 1:] | bad[1:, 1:]
+    assert np.array_equal(got[~touched], want[~touched])
+
+
 def test_residues_vanish_on_consistent_phase(torch_cuda):
     nr, nc = 40, 50
     t = 0.3 * np.arange(nc)[None, :] + 0.2 * np.arange(nr)[:, None]
