@@ -927,12 +927,7 @@ static cudaStream_t lib_stream(int dev)
 template <typename T>
 static T *dev_alloc_async(size_t n, cudaStream_t s)
 {
-    T *p = nullptr;
-    if (cudaMallocAsync((void **)&p, (n ? n : 1) * sizeof(T), s) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return p;
+    return static_cast<T *>(pool_alloc((n ? n : 1) * sizeof(T), s));
 }
 
 }  // namespace cuphu
@@ -1576,7 +1571,11 @@ static int build_costs_launcher(const float *d_phase, const float *d_corr, const
     if (d_roww) {
         /* the launcher interface passes two weight arrays; the kernel reads
          * one flat array, so gather them once */
-        CUPHU_TRY_CUDA(cudaMallocAsync((void **)&w, (nra + nca) * sizeof(short) + 8, s));
+        w = static_cast<short *>(pool_alloc((nra + nca) * sizeof(short) + 8, s));
+        if (!w) {
+            cudaFreeAsync(out, s);
+            return fail(CUPHU_ERR_ALLOC, "device allocation failed");
+        }
         CUPHU_TRY_CUDA(cudaMemcpyAsync(w, d_roww, nra * sizeof(short), cudaMemcpyDeviceToDevice, s));
         CUPHU_TRY_CUDA(cudaMemcpyAsync(w + nra, d_colw, nca * sizeof(short), cudaMemcpyDeviceToDevice, s));
     }
@@ -1942,6 +1941,7 @@ int cuphu_release_workspace(int gpu_id)
         W.dev = nullptr;
         W.host = nullptr;
         W.dev_size = W.host_size = 0;
+        pool_trim(gpu_id);
     }
     cudaSetDevice(prev);
     return rc;

@@ -474,11 +474,8 @@ int run_bridge(float *unw, uint32_t *cc, const unsigned char *mask, int nrow, in
     if (n < 2) return 0;
     std::vector<void *> owned;
     auto take = [&](size_t bytes) -> void * {
-        void *p = nullptr;
-        if (cudaMallocAsync(&p, std::max<size_t>(bytes, 16), s) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
+        void *p = pool_alloc(std::max<size_t>(bytes, 16), s);
+        if (!p) return nullptr;
         owned.push_back(p);
         return p;
     };

@@ -92,6 +92,12 @@ struct CostConsts {
 
 CostConsts make_cost_consts(const CuPhuParams &p);
 
+/* pool.cu: stream-ordered device memory of the library's own pool on the
+ * current device (NULL when out of memory); free it with cudaFreeAsync.
+ * pool_trim gives the idle memory back. */
+void *pool_alloc(size_t bytes, cudaStream_t s);
+void pool_trim(int dev);
+
 /* ── error plumbing ─────────────────────────────────────────────────────── */
 void set_error(const std::string &msg);
 int fail(int code, const std::string &msg);

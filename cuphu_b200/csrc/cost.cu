@@ -982,11 +982,11 @@ static int launch_costs7_all(const float *ph, const float *corr, const short *we
     /* scratch: the queue counter, the laycost table (DEFO), the queue */
     constexpr size_t kTabOff = 256, kQueueOff = kTabOff + kC7Tab * sizeof(short);
     static_assert(kQueueOff % 256 == 0, "queue offset");
-    void *buf = nullptr;
+    void *buf = pool_alloc((size_t)cap * sizeof(C7Global) + kQueueOff, s);
     C7Global *gq = nullptr;
     unsigned *gqn = nullptr;
     short *laytab = nullptr;
-    if (cudaMallocAsync(&buf, (size_t)cap * sizeof(C7Global) + kQueueOff, s) == cudaSuccess) {
+    if (buf) {
         gqn = reinterpret_cast<unsigned *>(buf);
         gq = reinterpret_cast<C7Global *>(static_cast<char *>(buf) + kQueueOff);
         CUPHU_TRY_CUDA(cudaMemsetAsync(gqn, 0, sizeof(unsigned), s));
@@ -995,8 +995,6 @@ static int launch_costs7_all(const float *ph, const float *corr, const short *we
             k_c7_laytab<<<kC7Tab / 256, 256, 0, s>>>(laytab, k);
             CUPHU_TRY_CUDA(cudaGetLastError());
         }
-    } else {
-        cudaGetLastError();
     }
     int rc = launch_costs7_t<DEFO, 0>(ph, corr, weights, nrow, ncol, k, costs, gq, gqn, cap, laytab,
                                       s);
