@@ -367,7 +367,9 @@ struct SolverJob {
         sp.skip_block = solver_take_skip_block(dev);
         sp.pass_iters = d_pass;
         int rc = 0;
-        if (res.nblk) rc = launch_resident(res, d_tiles, P, d_ctl, sp, s);
+        if (res.nblk)
+            rc = fp64 ? launch_resident_fp64(res, d_tiles, P, d_ctl, sp, s)
+                      : launch_resident_mixed(res, d_tiles, P, d_ctl, sp, s);
         if (!rc && !stream.empty())
             rc = launch_solve(fp64, d_stream, d_item, stream_items, (int)stream.size(), P, pitch,
                               rows, d_st, d_part, d_ctl, sp, dev, s);
@@ -476,11 +478,7 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     int nsm = 0;
     CUPHU_TRY_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     tune_note_items(0);
-    if (jo.fp64) {
-        for (int t = 0; t < ntiles; ++t) SJ.plan.streamed.push_back(t);
-    } else {
-        plan_resident(pl.tiles, nsm, SJ.plan);
-    }
+    plan_resident(pl.tiles, nsm, jo.fp64, SJ.plan);
     const size_t nsched = SJ.plan.sched.size(), nstream = SJ.plan.streamed.size();
     const size_t nps = nstream ? np : 0;
 
@@ -526,11 +524,11 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
         P.x = b.take<double>(np);
         P.dx = jo.fp64 || !nstream ? nullptr : b.take<float>(np);
         P.bvec = jo.fp64 ? nullptr : b.take<double>(np);
-        P.r = b.take<char>(nps * vs);
+        P.r = b.take<char>((jo.fp64 ? np : nps) * vs);
         P.p0 = b.take<char>(nps * vs);
         P.p1 = b.take<char>(nps * vs);
         P.q = b.take<char>(nps * vs);
-        P.diag = b.take<char>(jo.fp64 ? nps * vs : 0);
+        P.diag = b.take<char>(jo.fp64 ? np * vs : 0);
         P.z = b.take<char>(np * vs);
         P.q1 = jo.fp64 ? nullptr : b.take<float>(nps);
         P.unw = b.take<float>(np);
@@ -571,7 +569,7 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
         d_post = post_bytes ? b.take<char>(post_bytes) : nullptr;
         d_shift = b.take<SceneOut>(nsc);
         d_bars = b.take<unsigned>(nsched);
-        d_rim = b.take<char>(resident_rim_bytes(SJ.plan.nblk));
+        d_rim = b.take<char>(resident_rim_bytes(SJ.plan.nblk, jo.fp64));
         d_mail = b.take<char>(resident_mail_bytes(SJ.plan.nblk));
         d_ccbuf = cc_bytes ? b.take<char>(cc_bytes) : nullptr;
     };

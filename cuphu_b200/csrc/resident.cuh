@@ -1,5 +1,6 @@
 /*
- * resident.cuh -- host interface of the on-chip Laplace solver (resident.cu).
+ * resident.cuh -- host interface of the on-chip Laplace solver: resident.cu
+ * (mixed precision), resident_fp64.cu, and the plan (resident_plan.cu).
  */
 #pragma once
 
@@ -9,8 +10,9 @@
 
 namespace cuphu {
 
-constexpr int kResItems = 14;      /* work items a block can hold */
-constexpr int kResMaxG = 7;        /* largest group: 2^7 blocks   */
+constexpr int kResItemsMixed = 14;  /* work items a block can hold */
+constexpr int kResItems64 = 8;
+constexpr int kResMaxG = 7;         /* largest group: 2^7 blocks   */
 constexpr int kResMembers = 1 << kResMaxG;
 
 struct ResTile { int tile, g, nact, phys0; };   /* a scheduled tile: group of 2^g members,
@@ -39,11 +41,12 @@ struct ResidentArgs {                   /* the plan on the device, and scratch *
     int nblk = 0;
 };
 
-bool resident_fits(int nitems);
-void plan_resident(const std::vector<TileDesc> &tiles, int nblk, ResidentPlan &R);
-size_t resident_rim_bytes(int nblk);
+void plan_resident(const std::vector<TileDesc> &tiles, int nblk, bool fp64, ResidentPlan &R);
+size_t resident_rim_bytes(int nblk, bool fp64);
 size_t resident_mail_bytes(int nblk);
-int launch_resident(const ResidentArgs &A, const TileDesc *tiles, const SolverPlanes &P,
-                    SolverCtl *ctl, const SolveParams &sp, cudaStream_t s);
+int launch_resident_mixed(const ResidentArgs &A, const TileDesc *tiles, const SolverPlanes &P,
+                          SolverCtl *ctl, const SolveParams &sp, cudaStream_t s);
+int launch_resident_fp64(const ResidentArgs &A, const TileDesc *tiles, const SolverPlanes &P,
+                         SolverCtl *ctl, const SolveParams &sp, cudaStream_t s);
 
 }  // namespace cuphu

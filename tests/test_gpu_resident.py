@@ -1,16 +1,17 @@
-"""The on-chip solver (mixed precision, tiles that fit the chip) at the sizes
-where its split can go wrong: single rows and columns, items exactly filled
+"""The on-chip solvers (tiles that fit the chip, both precisions) at the sizes
+where their split can go wrong: single rows and columns, items exactly filled
 and one pixel over, groups with idle members, ragged last levels, the largest
-tile it takes and the first one it leaves to the streaming solver.  The
-reference is the FP64 streaming solve of the same tile, which the other tests
-pin to the oracle bit for bit.  The bounds are those of the mixed mode
-elsewhere: 1e-3 rad RMS of the continuous solution and 1e-4 of the cycles,
-with the floor of 3 that a handful of half-cycle pixels needs."""
+tiles they take and the first one they leave to the streaming solver.  FP64 is
+compared with the CPU oracle bit for bit; mixed precision with FP64, within
+the bounds of the mixed mode elsewhere: 1e-3 rad RMS of the continuous
+solution and 1e-4 of the cycles, with the floor of 3 that a handful of
+half-cycle pixels needs."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
+import oracle as O
 from cuphu_b200 import synthetic as S
 from cuphu_b200._lib import (CuPhuScene, CuPhuSolveStats, check, default_params,
                              default_solve_options, lib)
@@ -89,3 +90,33 @@ def test_batch_of_on_chip_and_streamed_tiles(torch_cuda):
         assert np.array_equal(got[i][0].view(np.int32), want[0][0].view(np.int32))
         assert np.array_equal(got[i][1], want[0][1])
     assert st.max_iters_pass == longest
+
+
+@pytest.mark.parametrize("shape,blocked", [
+    ((1, 1), False), ((1, 70), False), ((70, 1), False), ((16, 64), True), ((17, 65), False),
+    ((15, 1037), True), ((1025, 63), False), ((500, 333), True), ((1024, 1024), False)])
+def test_fp64_on_chip_solve_bit_exact_vs_oracle(torch_cuda, shape, blocked):
+    costs, ph = scene(*shape, seed=5 + shape[0] + 3 * shape[1], blocked=blocked)
+    x, k, unw, iters = O.laplace_f64(costs, ph, O.lap_opts(n_irls=1, max_iter=60))
+    gu, gk, gc, st = gpu_solve(torch_cuda, costs, ph, precision=1, n_irls=1, max_iter=60)
+    assert st.total_iters == int(iters.sum())
+    assert np.array_equal(gk, k)
+    assert np.array_equal(gu.view(np.int32), unw.view(np.int32))
+    assert np.array_equal(gc, (x + (float(ph[0, 0]) - x[0, 0])).astype(np.float32))
+
+
+def test_fp64_division_outside_the_correction_range(torch_cuda):
+    """Weights of 2^60 and 2^120: the diagonals of the first allow the
+    correction steps, those of the second take the IEEE division.  Everything
+    scales by powers of two (eps is far below both), so the solutions agree
+    bit for bit."""
+    from cuphu_b200.autograd import wls_solve
+    t = torch_cuda
+    g = t.Generator(device="cuda")
+    g.manual_seed(3)
+    gd, gr, w = (t.rand((90, 75), generator=g, device="cuda") for _ in range(3))
+    w = (w * 3 + 0.5)
+    out = [wls_solve(gd, gr, w * 2.0 ** e, w.flip(0).contiguous() * 2.0 ** e, max_iter=40)
+           for e in (60, 120)]
+    assert t.isfinite(out[0]).all() and float(out[0].abs().max()) > 0
+    assert t.equal(out[0], out[1])
