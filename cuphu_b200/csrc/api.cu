@@ -570,7 +570,7 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
         d_shift = b.take<SceneOut>(nsc);
         d_bars = b.take<unsigned>(nsched);
         d_rim = b.take<char>(resident_rim_bytes(SJ.plan.nblk, jo.fp64));
-        d_mail = b.take<char>(resident_mail_bytes(SJ.plan.nblk));
+        d_mail = b.take<char>(resident_mail_bytes(SJ.plan.nblk, jo.fp64));
         d_ccbuf = cc_bytes ? b.take<char>(cc_bytes) : nullptr;
     };
     SolverPlanes P = {};

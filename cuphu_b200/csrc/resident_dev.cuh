@@ -1,12 +1,9 @@
 /*
  * resident_dev.cuh -- what the two on-chip solver kernels (resident.cu: mixed
  * precision, resident_fp64.cu) share: the block's shared state, packets,
- * tensor memory, bounded waits, the group's barrier and geometry, and the
- * exchange of partial sums.  A kernel's file defines kResItems (items of a
- * block) and kResCols (TMEM columns of an item) before it includes this; all
- * of it has internal linkage.
+ * tensor memory, bounded waits, the group's barrier, and the launch.  A kernel's file defines ResOwn (its own part of the shared state)
+ * before it includes this; all of it has internal linkage.
  */
-#include "resident_geom.cuh"
 #include "solver.cuh"
 
 #include <cuda/atomic>
@@ -16,16 +13,7 @@ namespace {
 
 constexpr int kResEngines = 2;                          /* 256-thread engines per block */
 constexpr int kResThreads = kResEngines * kItemThreads;
-constexpr int kResPerEngine = kResItems / kResEngines;
-constexpr int kRim = 2 * kItemBx + 2 * kItemBy;         /* halo pixels of an item */
-constexpr int kPnW = kItemBx + 8;                       /* p row: 4 columns each side */
-constexpr int kPnN = (kItemBy + 2) * kPnW;
-constexpr int kWdN = (kItemBy + 1) * kItemBx;           /* down arcs, one row above */
-constexpr int kWrW2 = kItemBx + 4;                      /* right arcs, 4 columns left */
-constexpr int kWrN = kItemBy * kWrW2;
 constexpr int kTmemCols = 512;
-static_assert(2 * kResEngines * kResPerEngine * kResCols <= kTmemCols, "TMEM columns");
-
 /* The kernel's parameters. */
 struct ResParams {
     const TileDesc *tiles;
@@ -40,19 +28,15 @@ struct ResParams {
  * next to no L1, so a spilled word costs a trip to the L2. */
 struct ResShared {
     ResParams K;
-    double red[kResItems][kNComp][8];   /* warp sums per item and component */
-    double part[kNComp];                /* the block's partials */
-    double tot[kResThreads / 32][kNComp];   /* warp sums of an exchange */
+    ResOwn own;                         /* the kernel's own part */
     TileDesc T;
     TileState S;                        /* the tile's PCG scalars (thread 0) */
     unsigned *bar;                      /* barrier of the group */
-    unsigned bar_target, nact;
-    int g, member, nloc;                /* group of 2^g, this block's member, its items */
+    unsigned bar_target, nact;          /* blocks of the group */
+    int member, nloc;                   /* this block's member number and items */
     int skip;                           /* failure test: do not arrive at the next barrier */
-    unsigned nbr[kResItems][4];         /* packet base of the rim sources: above,
-                                           below, left, right (~0: outside) */
-    int li[kResItems];
-    unsigned short phys[kResMembers];
+    int li[kResItemsMixed];             /* the items, by number in the tile */
+    unsigned short phys[kResMaxBlocks]; /* the members' blocks */
     double alpha, beta;                 /* the mixed solve's are floats */
     int active, k;                      /* pass number of the IRLS pass's solve */
     unsigned seq;                       /* number of the last exchange */
@@ -194,179 +178,12 @@ __device__ __noinline__ bool group_sync(bool any_progress = false)
     return __syncthreads_and(ok);
 }
 
-/* A thread's view of its block. */
-struct ResCtx {
-    int eng, tid, warp, lane;
-    int rim_at, rim_nb, rim_pk;   /* this thread's rim pixel of an item: place in the p array
-                                     (-1: none), neighbour, packet */
-    uint32_t tm;           /* this thread's TMEM columns of its engine's first item */
-};
-
-__device__ __forceinline__ ResCtx make_ctx()
-{
-    const int warp = threadIdx.x >> 5;
-    const int eng = (int)threadIdx.x / kItemThreads, tid = (int)threadIdx.x % kItemThreads;
-    /* the halo ring of an item is the work of an engine's last 160 threads:
-     * the rows above and below (the neighbour's last and first row), the
-     * columns left and right (its last and first column) */
-    int rim_at = -1, rim_nb = 0, rim_pk = 0;
-    const int h = tid - (kItemThreads - kRim);
-    if (h >= 2 * kItemBx + kItemBy) {
-        const int r = h - 2 * kItemBx - kItemBy;
-        rim_at = (r + 1) * kPnW + 4 + kItemBx; rim_nb = 3; rim_pk = 2 * kItemBx + r;
-    } else if (h >= 2 * kItemBx) {
-        const int r = h - 2 * kItemBx;
-        rim_at = (r + 1) * kPnW + 3; rim_nb = 2; rim_pk = 2 * kItemBx + kItemBy + r;
-    } else if (h >= kItemBx) {
-        rim_at = (kItemBy + 1) * kPnW + 4 + h - kItemBx; rim_nb = 1; rim_pk = h - kItemBx;
-    } else if (h >= 0) {
-        rim_at = 4 + h; rim_nb = 0; rim_pk = kItemBx + h;
-    }
-    return ResCtx{eng, tid, warp, (int)threadIdx.x & 31, rim_at, rim_nb, rim_pk,
-                  res_shared().tmem + ((uint32_t)(warp & 3) << 21) +
-                      (uint32_t)(warp >> 2) * (kResPerEngine * kResCols)};
-}
-
-/* A block's mailbox: [parity][member m][component] packets, in the order in
- * which the threads read them (thread 32 w + 4 h + c: member 16 h + w,
- * component c). */
-constexpr int kMailN = 2 * kNComp * kResMembers;
-__device__ __forceinline__ ulonglong2 *mail_of(const ResCtx &C, int block, unsigned seq, int m, int c)
-{
-    return res_shared().K.A.mail + (size_t)block * kMailN + (seq & 1u) * (kNComp * kResMembers) +
-           ((m & 15) << 5) + ((m >> 4) << 2) + c;
-}
-
-/* The block's partials into sh.part: warp c forms the items' partials of
- * component c (lanes 2 i + h hold the half tree of warp parity h), then the
- * slot sums (items of a slot in order) and the butterfly levels inside the
- * block. */
-__device__ __forceinline__ void block_partials(const ResCtx &C, int ncomp)
-{
-    if (C.warp >= ncomp) return;
-    const int c = C.warp, i = C.lane >> 1, h = C.lane & 1;
-    double v = 0.0;
-    if (i < res_shared().nloc) {
-        const double *w = res_shared().red[i][c];
-        v = (w[h] + w[h + 4]) + (w[h + 2] + w[h + 6]);
-    }
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    const int slog = 8 - res_shared().g, S = 1 << slog, sub = C.lane & (S - 1);
-    double a = 0.0;
-    for (int k = 0; k < res_shared().nloc; k += S) {
-        const double x = __shfl_sync(0xffffffffu, v, (2 * (k + sub)) & 31);
-        if (k + sub < res_shared().nloc) a += x;
-    }
-    for (int off = S >> 1; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-    if (C.lane == 0) res_shared().part[c] = a;
-}
-
-/* Send the block's partials to every block of the group and ask for nothing
- * yet: thread 4 d + c stores component c into member d's mailbox. */
-__device__ __forceinline__ void send_partials(const ResCtx &C, int ncomp, unsigned seq)
-{
-    static_assert(kResThreads == kNComp * kResMembers, "one packet per thread");
-    __syncthreads();
-    const int d = threadIdx.x >> 2, c = threadIdx.x & 3;
-    if (c < ncomp && d < (1 << res_shared().g)) {
-        const unsigned ph = res_shared().phys[d];
-        if (ph != 0xffffu)
-            packet_store(mail_of(C, ph, seq, res_shared().member, c),
-                         (unsigned long long)__double_as_longlong(res_shared().part[c]),
-                         (unsigned long long)seq);
-    }
-}
-
-/* Wait for exchange `seq` and finish the tree; the totals are returned in warp
- * 0.  One hop: every member stores its packets into every mailbox (8 KB per
- * block and exchange), and a thread polls one packet of its own block's
- * mailbox.  Measured for 128 blocks, from the stores to the totals: 1900 cycles,
- * against 4900 when one block per component collects and publishes (two
- * hops) and 7500 when every block polls the members' own copies (128 readers
- * of each line).  The members' bits combine
- * from the top: three levels across the lanes, four across the warps. */
-template <int NCOMP>
-__device__ __forceinline__ bool totals(const ResCtx &C, unsigned seq, double out[NCOMP])
-{
-    const int c = C.lane & 3, m = ((C.lane >> 2) << 4) | C.warp;
-    unsigned long long lo = 0;
-    bool ok = true;
-    if (c < NCOMP && m < (1 << res_shared().g) && res_shared().phys[m] != 0xffffu) {
-        const ulonglong2 *p = mail_of(C, blockIdx.x, seq, m, c);
-        unsigned long long hi;
-        packet_load(p, lo, hi);
-        if (hi != (unsigned long long)seq) {
-            Waiter w(res_shared().K.ctl, res_shared().K.sp.timeout_ns);
-            do {
-                if (!w.turn()) {
-                    ok = false;
-                    break;
-                }
-                packet_load(p, lo, hi);
-            } while (hi != (unsigned long long)seq);
-        }
-    }
-    __syncwarp();
-    double v = __longlong_as_double((long long)lo);
-#pragma unroll
-    for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (C.lane < NCOMP) res_shared().tot[C.warp][C.lane] = v;
-    ok = __syncthreads_and(ok);
-    if (C.warp == 0) {
-        const int k = C.lane >> 2;
-        v = c < NCOMP ? res_shared().tot[k][c] + res_shared().tot[k + 8][c] : 0.0;
-#pragma unroll
-        for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-#pragma unroll
-        for (int j = 0; j < NCOMP; ++j) out[j] = __shfl_sync(0xffffffffu, v, j);
-    }
-    return ok;
-}
-
-/* void the k-th rim packet of this block (each kernel has its own kind) */
-__device__ __forceinline__ void rim_void(int k);
-
-/* this block's items of the tile, their rim sources; the packets of an
- * earlier tile are voided */
-__device__ __noinline__ void setup_items()
-{
-    ResShared &sh = res_shared();
-    const ResParams &K = sh.K;
-    const TileDesc &T = sh.T;
-    if (threadIdx.x < kResItems) {
-        const int i = threadIdx.x, slog = 8 - sh.g;
-        const int u = ((i & ((1 << slog) - 1)) << sh.g) | sh.member;
-        const int li = 256 * (i >> slog) + res_slot(u);
-        sh.li[i] = li;
-        if (i < sh.nloc) {
-            const int row = li / T.nbx, col = li % T.nbx;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                int n = -1;
-                if (k == 0 && row > 0) n = li - T.nbx;
-                if (k == 1 && li + T.nbx < T.nitems) n = li + T.nbx;
-                if (k == 2 && col > 0) n = li - 1;
-                if (k == 3 && col + 1 < T.nbx) n = li + 1;
-                unsigned base = ~0u;
-                if (n >= 0) {
-                    const int v = res_u(n & 255), m = v & ((1 << sh.g) - 1);
-                    base = ((unsigned)sh.phys[m] * kResItems + ((n >> 8) << slog) + (v >> sh.g)) *
-                           2 * kRim;
-                }
-                sh.nbr[i][k] = base;
-            }
-        }
-    }
-    for (int k = threadIdx.x; k < sh.nloc * 2 * kRim; k += kResThreads)
-        rim_void(k);
-    for (int k = threadIdx.x; k < kMailN; k += kResThreads)
-        packet_store(K.A.mail + (size_t)blockIdx.x * kMailN + k, 0ull, 0ull);
-    if (threadIdx.x == 0) sh.seq = 0u;
-}
-
 /* The body of both kernels: take tensor memory, run this block's part of its
- * tiles in order, give the tensor memory back. */
-template <typename Run> __device__ __forceinline__ void resident_blocks(const ResParams &K, Run run)
+ * tiles in order, give the tensor memory back.  begin(R) sets the kernel's
+ * own part for a tile (one thread); run() returns false when a wait ran
+ * out. */
+template <typename Begin, typename Run>
+__device__ __forceinline__ void resident_blocks(const ResParams &K, Begin begin, Run run)
 {
     ResShared &sh = res_shared();
     for (int k = threadIdx.x; k < (int)(sizeof(ResParams) / 4); k += kResThreads)
@@ -387,16 +204,15 @@ template <typename Run> __device__ __forceinline__ void resident_blocks(const Re
         const ResWork W = K.A.work[w];
         const ResTile R = K.A.sched[W.sched];
         __syncthreads();   /* the last tile's reads of sh are done */
-        for (int k = threadIdx.x; k < (1 << R.g); k += kResThreads)
+        for (int k = threadIdx.x; k < R.nmem; k += kResThreads)
             sh.phys[k] = K.A.phys[R.phys0 + k];
         if (threadIdx.x == 0) {
             sh.T = K.tiles[R.tile];
             sh.bar = K.A.bars + W.sched;
             sh.bar_target = 0u;
             sh.nact = (unsigned)R.nact;
-            sh.g = R.g;
             sh.member = W.member;
-            sh.nloc = res_count(sh.T.nitems, W.member, R.g);
+            begin(R);
             sh.skip = w == w0 && (int)blockIdx.x == K.sp.skip_block;
         }
         __syncthreads();

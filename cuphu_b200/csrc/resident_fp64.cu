@@ -16,13 +16,33 @@
  * rounds correctly (P. Markstein, "Computation of elementary functions on the
  * IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1), 1990): five
  * FP64 operations in place of a division of some thirty.
+ *
+ * The split is by the slots of k_solve's reduction tree, so that the sums are
+ * k_solve's to the bit: sums items j, j + 256, ... per slot j, then the 256
+ * slots by a butterfly over the slot's lane bits (16, 8, 4, 2, 1) and its
+ * warp bits (4, 2, 1).  A group of 2^g blocks deals the slots out so that
+ * the first 8 - g levels of that butterfly stay inside a block: a block
+ * publishes one partial, and every block finishes the tree for itself.
+ *
+ * What bounds it: two exchanges of about 2.5 us each per iteration (see
+ * resident.cu), and with 8 items per block the shared-memory and tensor-memory
+ * latency of the two halves.  Per iteration 6.8 us at 256 x 256, 8.7 us at
+ * 512 x 512, 14.2 us at 967 x 967; the streaming form took 22, 28 and 50 us.
  */
-#include "resident.cuh"
+#include "resident_geom.cuh"
 
 namespace cuphu {
 namespace {
 constexpr int kResItems = kResItems64;
-constexpr int kResCols = 32;   /* x, r, diag and 1/diag of four pixels */
+struct ResOwn {
+    double red[kResItems][8];           /* warp sums per item */
+    double part;                        /* the block's partial */
+    double tot[16];                     /* warp sums of an exchange */
+    unsigned nbr[kResItems][4];         /* packet base of the rim sources: above,
+                                           below, left, right (~0: outside) */
+    int g;                              /* group of 2^g members */
+    int slow;                           /* some quotient of the block needs IEEE divisions */
+};
 }  // namespace
 }  // namespace cuphu
 #include "resident_dev.cuh"
@@ -30,9 +50,63 @@ constexpr int kResCols = 32;   /* x, r, diag and 1/diag of four pixels */
 namespace cuphu {
 namespace {
 
+constexpr int kResCols = 32;   /* TMEM columns of an item: x, r, diag and 1/diag of four pixels */
+constexpr int kResPerEngine = kResItems / kResEngines;
+constexpr int kRim = 2 * kItemBx + 2 * kItemBy;         /* halo pixels of an item */
+/* Rows of an item's arrays: the first two of every thread's four pixels, then
+ * the other two (so a warp reads 16-byte pieces without bank conflicts; four
+ * doubles in place cost two passes per read), then the halo columns: p has
+ * one on each side, the right arcs one on the left. */
+constexpr int kPnW = kItemBx + 2;
+constexpr int kPnN = (kItemBy + 2) * kPnW;
+constexpr int kWdN = (kItemBy + 1) * kItemBx;           /* down arcs, one row above */
+constexpr int kWrW = kItemBx + 2;
+constexpr int kWrN = kItemBy * kWrW;
+constexpr int kHalf = kItemBx / 2, kLeft = kItemBx, kRight = kItemBx + 1;
+__device__ __forceinline__ int col_at(int c)            /* place of column c in a row */
+{
+    return ((c >> 1) & 1) * kHalf + (c >> 2) * 2 + (c & 1);
+}
+static_assert(2 * kResEngines * kResPerEngine * kResCols <= kTmemCols, "TMEM columns");
 constexpr int kResItemD = kPnN + kWdN + kWrN;   /* doubles of an item */
 constexpr size_t kResSmem = (size_t)kResItems * kResItemD * 8 + kResSharedB;
 static_assert(kResSmem <= 232448, "shared memory of a block");
+
+/* A thread's view of its block. */
+struct ResCtx {
+    int eng, tid, warp, lane;
+    int rim_at, rim_nb, rim_pk;   /* this thread's rim pixel of an item: place in the p array
+                                     (-1: none), neighbour, packet */
+    int rim_r, rim_c;             /* its row and column in the item (-1 .. 16, -1 .. 64) */
+    uint32_t tm;           /* this thread's TMEM columns of its engine's first item */
+};
+
+__device__ __forceinline__ ResCtx make_ctx()
+{
+    const int warp = threadIdx.x >> 5;
+    const int eng = (int)threadIdx.x / kItemThreads, tid = (int)threadIdx.x % kItemThreads;
+    /* the halo ring of an item is the work of an engine's last 160 threads:
+     * the rows above and below (the neighbour's last and first row), the
+     * columns left and right (its last and first column) */
+    int rim_at = -1, rim_nb = 0, rim_pk = 0, rim_r = 0, rim_c = 0;
+    const int h = tid - (kItemThreads - kRim);
+    if (h >= 2 * kItemBx + kItemBy) {
+        rim_r = h - 2 * kItemBx - kItemBy; rim_c = kItemBx;
+        rim_at = (rim_r + 1) * kPnW + kRight; rim_nb = 3; rim_pk = 2 * kItemBx + rim_r;
+    } else if (h >= 2 * kItemBx) {
+        rim_r = h - 2 * kItemBx; rim_c = -1;
+        rim_at = (rim_r + 1) * kPnW + kLeft; rim_nb = 2; rim_pk = 2 * kItemBx + kItemBy + rim_r;
+    } else if (h >= kItemBx) {
+        rim_r = kItemBy; rim_c = h - kItemBx;
+        rim_at = (kItemBy + 1) * kPnW + col_at(rim_c); rim_nb = 1; rim_pk = rim_c;
+    } else if (h >= 0) {
+        rim_r = -1; rim_c = h;
+        rim_at = col_at(h); rim_nb = 0; rim_pk = kItemBx + h;
+    }
+    return ResCtx{eng, tid, warp, (int)threadIdx.x & 31, rim_at, rim_nb, rim_pk, rim_r, rim_c,
+                  res_shared().tmem + ((uint32_t)(warp & 3) << 21) +
+                      (uint32_t)(warp >> 2) * (kResPerEngine * kResCols)};
+}
 
 __device__ __forceinline__ double *pn_of(int i)
 {
@@ -44,8 +118,9 @@ __device__ __forceinline__ uint32_t tm_of(const ResCtx &C, int i)
 {
     return C.tm + (uint32_t)(i / kResEngines) * kResCols;
 }
-/* columns of an item */
-constexpr int kTmX = 0, kTmR = 8, kTmD = 16, kTmY = 24;
+/* columns of an item: x, r, diag and 1/diag (4 each) of the first two pixels,
+ * then of the other two */
+constexpr int kTmHalf = 16;
 
 /* rim packets: z of a pixel and the exchange number */
 __device__ __forceinline__ ulonglong2 *rim_at(unsigned base)
@@ -61,39 +136,194 @@ __device__ __forceinline__ void rim_void(int k)
     rim_store(rim_at(blockIdx.x * kResItems * 2 * kRim + k), 0.0, 0u);
 }
 
-__device__ __forceinline__ void unpack4(const uint32_t *t, double v[4])
+__device__ __forceinline__ void unpack2(const uint32_t *t, double v[2])
 {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = __hiloint2double((int)t[2 * j + 1], (int)t[2 * j]);
+    v[0] = __hiloint2double((int)t[1], (int)t[0]);
+    v[1] = __hiloint2double((int)t[3], (int)t[2]);
 }
-__device__ __forceinline__ void tm_st4d(uint32_t a, const double v[4])
+__device__ __forceinline__ void pack2(const double v[2], float *f)
 {
-    float f[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
         f[2 * j] = __int_as_float(__double2loint(v[j]));
         f[2 * j + 1] = __int_as_float(__double2hiint(v[j]));
     }
-    tm_st8(a, f);
 }
-__device__ __forceinline__ void lds4(const double *p, double v[4])
+__device__ __forceinline__ void lds2(const double *p, double v[2])
 {
-    const double2 a = reinterpret_cast<const double2 *>(p)[0];
-    const double2 b = reinterpret_cast<const double2 *>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    const double2 a = *reinterpret_cast<const double2 *>(p);
+    v[0] = a.x; v[1] = a.y;
+}
+__device__ __forceinline__ void sts2(double *p, const double v[2])
+{
+    *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
 }
 
 /* r / d from y = RN(1/d).  The correction steps are exact where nothing
- * underflows or overflows; a residual outside [2^-900, 2^900] and a diagonal
- * outside [2^-100, 2^100] (y = 0 marks it) take the IEEE division. */
+ * underflows or overflows: for a residual that is zero or in [2^-900, 2^900]
+ * (res_odd tests the rest) and a diagonal in [2^-100, 2^100] (y = 0 marks the
+ * rest).  A block that meets another value forms its quotients with IEEE
+ * divisions, in functions of their own (slow_fold, slow_update): a division
+ * in the iterations would be a call there, and cost them their registers. */
 __device__ __forceinline__ double quotient(double r, double d, double y)
 {
     const double q0 = __dmul_rn(r, y);
     const double q1 = __fma_rn(__fma_rn(-q0, d, r), y, q0);
-    double q = __fma_rn(__fma_rn(-q1, d, r), y, q1);
+    return __fma_rn(__fma_rn(-q1, d, r), y, q1);
+}
+__device__ __forceinline__ bool res_odd(double r)
+{
     const unsigned e = ((unsigned)__double2hiint(r) & 0x7fffffffu) - (123u << 20);
-    if ((e > (1800u << 20) || __double2hiint(y) == 0) && r != 0.0) q = __ddiv_rn(r, d);
-    return q;
+    return e > (1800u << 20) && r != 0.0;
+}
+
+/* a / b rounded to nearest for a, b > 0, without the call that the division
+ * operator can make (a call in the iterations would push q = A p out of the
+ * registers): the reciprocal by Newton steps from the hardware's
+ * approximation, then Markstein's two correction steps.  Operands outside
+ * [2^-900, 2^900] are scaled by 2^+-600 first; a result that is not a normal
+ * number may differ from the operator's in its last bit. */
+__device__ __forceinline__ double quotient_pos(double a, double b)
+{
+    auto scale = [](double v) {
+        const int e = (__double2hiint(v) >> 20) & 0x7ff;
+        return e < 123 ? 0x1p600 : e > 1923 ? 0x1p-600 : 1.0;
+    };
+    const double sa = scale(a), sb = scale(b);
+    a *= sa;
+    b *= sb;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    const double q = quotient(a, b, y);
+    const double back = sa == 1.0 ? 1.0 : sa > 1.0 ? 0x1p-600 : 0x1p600;   /* 1 / sa */
+    return (q * back) * sb;
+}
+
+/* A block's mailbox: [parity][member m] packets, 64 bytes apart: two writers
+ * in one 32-byte sector cost an iteration at 512^2 1.3 us */
+constexpr int kMailStep = 4;
+constexpr int kMailN = 2 * kResMembers * kMailStep;
+__device__ __forceinline__ ulonglong2 *mail_of(int block, unsigned seq, int m)
+{
+    return res_shared().K.A.mail + (size_t)block * kMailN + ((seq & 1u) * kResMembers + m) * kMailStep;
+}
+
+/* The block's partial into own.part: warp 0 forms the items' partials (lanes
+ * 2 i + h hold the half tree of warp parity h), then the slot sums (items of
+ * a slot in order) and the butterfly levels inside the block. */
+__device__ __forceinline__ void block_partial(const ResCtx &C)
+{
+    if (C.warp != 0) return;
+    ResOwn &own = res_shared().own;
+    const int i = C.lane >> 1, h = C.lane & 1, nloc = res_shared().nloc;
+    double v = 0.0;
+    if (i < nloc) {
+        const double *w = own.red[i];
+        v = (w[h] + w[h + 4]) + (w[h + 2] + w[h + 6]);
+    }
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    const int slog = 8 - own.g, S = 1 << slog, sub = C.lane & (S - 1);
+    double a = 0.0;
+    for (int k = 0; k < nloc; k += S) {
+        const double x = __shfl_sync(0xffffffffu, v, (2 * (k + sub)) & 31);
+        if (k + sub < nloc) a += x;
+    }
+    for (int off = S >> 1; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+    if (C.lane == 0) own.part = a;
+}
+
+/* Send the block's partial to every block of the group: thread 4 d to member
+ * d's mailbox (spread over all warps: a warp's store goes to eight blocks). */
+__device__ __forceinline__ void send_partial(unsigned seq)
+{
+    __syncthreads();
+    const ResShared &sh = res_shared();
+    const int d = threadIdx.x >> 2;
+    if ((threadIdx.x & 3) == 0 && d < (1 << sh.own.g) && sh.phys[d] != 0xffffu)
+        packet_store(mail_of(sh.phys[d], seq, sh.member),
+                     (unsigned long long)__double_as_longlong(sh.own.part),
+                     (unsigned long long)seq);
+}
+
+/* Wait for exchange `seq` and finish the tree; the total is returned in warp
+ * 0.  One hop: every member stores its packet into every mailbox, and thread
+ * 32 w + 4 h polls the packet of member 16 h + w of its own block's mailbox.
+ * The members' bits combine from the top: three levels across the lanes,
+ * four across the warps. */
+__device__ __forceinline__ bool total(const ResCtx &C, unsigned seq, double &out)
+{
+    ResShared &sh = res_shared();
+    bool ok = true;
+    const int m = ((C.lane >> 2) << 4) | C.warp;
+    unsigned long long lo = 0;
+    if ((C.lane & 3) == 0 && m < (1 << sh.own.g) && sh.phys[m] != 0xffffu) {
+        const ulonglong2 *p = mail_of(blockIdx.x, seq, m);
+        unsigned long long hi;
+        packet_load(p, lo, hi);
+        if (hi != (unsigned long long)seq) {
+            Waiter w(sh.K.ctl, sh.K.sp.timeout_ns);
+            do {
+                if (!w.turn()) {
+                    ok = false;
+                    break;
+                }
+                packet_load(p, lo, hi);
+            } while (hi != (unsigned long long)seq);
+        }
+    }
+    __syncwarp();
+    double v = __longlong_as_double((long long)lo);
+#pragma unroll
+    for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (C.lane == 0) sh.own.tot[C.warp] = v;
+    ok = __syncthreads_and(ok);
+    if (C.warp == 0) {
+        v = C.lane < 16 ? sh.own.tot[C.lane] : 0.0;
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        out = v;
+    }
+    return ok;
+}
+
+/* this block's items of the tile, their rim sources; the packets of an
+ * earlier tile are voided */
+__device__ __noinline__ void setup_items()
+{
+    ResShared &sh = res_shared();
+    const ResParams &K = sh.K;
+    const TileDesc &T = sh.T;
+    if (threadIdx.x < kResItems) {
+        const int i = threadIdx.x, slog = 8 - sh.own.g;
+        const int u = ((i & ((1 << slog) - 1)) << sh.own.g) | sh.member;
+        const int li = 256 * (i >> slog) + res_slot(u);
+        sh.li[i] = li;
+        if (i < sh.nloc) {
+            const int row = li / T.nbx, col = li % T.nbx;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                int n = -1;
+                if (k == 0 && row > 0) n = li - T.nbx;
+                if (k == 1 && li + T.nbx < T.nitems) n = li + T.nbx;
+                if (k == 2 && col > 0) n = li - 1;
+                if (k == 3 && col + 1 < T.nbx) n = li + 1;
+                unsigned base = ~0u;
+                if (n >= 0) {
+                    const int v = res_u(n & 255), m = v & ((1 << sh.own.g) - 1);
+                    base = ((unsigned)sh.phys[m] * kResItems + ((n >> 8) << slog) + (v >> sh.own.g)) *
+                           2 * kRim;
+                }
+                sh.own.nbr[i][k] = base;
+            }
+        }
+    }
+    for (int k = threadIdx.x; k < sh.nloc * 2 * kRim; k += kResThreads)
+        rim_void(k);
+    for (int k = threadIdx.x; k < kMailN; k += kResThreads)
+        packet_store(K.A.mail + (size_t)blockIdx.x * kMailN + k, 0ull, 0ull);
+    if (threadIdx.x == 0) sh.seq = 0u;
 }
 
 /* Load an item at the start of a pass: x, r and the diagonal from the planes,
@@ -106,6 +336,7 @@ __device__ __noinline__ void load_items()
     const SolverPlanes &P = sh.K.P;
     const TileDesc &T = sh.T;
     const int ty = C.tid / kItemTx, tx = C.tid % kItemTx;
+    bool odd = false;
     for (int i = C.eng; i < sh.nloc; i += kResEngines) {
         const int li = sh.li[i];
         const int r = (li / T.nbx) * kItemBy + ty, c0 = (li % T.nbx) * kItemBx + tx * kItemVx;
@@ -134,23 +365,33 @@ __device__ __noinline__ void load_items()
             }
             if (c0 + j >= T.nc - 1) wrt[j] = 0.f;
             yv[j] = dv[j] >= 0x1p-100 && dv[j] <= 0x1p100 ? __drcp_rn(dv[j]) : 0.0;
+            odd = odd || yv[j] == 0.0 || res_odd(rv[j]);
         }
         __syncwarp();
-        tm_st4d(tm_of(C, i) + kTmX, xv);
-        tm_st4d(tm_of(C, i) + kTmR, rv);
-        tm_st4d(tm_of(C, i) + kTmD, dv);
-        tm_st4d(tm_of(C, i) + kTmY, yv);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float f[16];
+            pack2(xv + 2 * h, f);
+            pack2(rv + 2 * h, f + 4);
+            pack2(dv + 2 * h, f + 8);
+            pack2(yv + 2 * h, f + 12);
+            tm_st8(tm_of(C, i) + h * kTmHalf, f);
+            tm_st8(tm_of(C, i) + h * kTmHalf + 8, f + 8);
+        }
         for (int k = C.tid; k < kPnN; k += kItemThreads) Pn[k] = 0.0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            WD[(ty + 1) * kItemBx + tx * kItemVx + j] = (double)wdn[j];
-            WR[ty * kWrW2 + 4 + tx * kItemVx + j] = (double)wrt[j];
-            if (ty == 0) WD[tx * kItemVx + j] = (double)up[j];
+            const int c = col_at(tx * kItemVx + j);
+            WD[(ty + 1) * kItemBx + c] = (double)wdn[j];
+            WR[ty * kWrW + c] = (double)wrt[j];
+            if (ty == 0) WD[c] = (double)up[j];
         }
-        if (tx == 0) WR[ty * kWrW2 + 3] = (double)lf;
+        if (tx == 0) WR[ty * kWrW + kLeft] = (double)lf;
         __syncwarp();
     }
     tm_wait_st();
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) res_shared().own.slow = odd;
     __syncthreads();
 }
 
@@ -161,10 +402,13 @@ __device__ __noinline__ void store_items()
     const ResShared &sh = res_shared();
     const TileDesc &T = sh.T;
     for (int i = C.eng; i < sh.nloc; i += kResEngines) {
-        uint32_t t[8];
-        tm_ld8(tm_of(C, i) + kTmX, t);
         double xv[4];
-        unpack4(t, xv);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t t[8];
+            tm_ld8(tm_of(C, i) + h * kTmHalf, t);
+            unpack2(t, xv + 2 * h);
+        }
         const int li = sh.li[i];
         const int r = (li / T.nbx) * kItemBy + C.tid / kItemTx;
         const int c0 = (li % T.nbx) * kItemBx + (C.tid % kItemTx) * kItemVx;
@@ -178,7 +422,7 @@ __device__ __forceinline__ void item_sum(const ResCtx &C, int i, double v)
 {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (C.lane == 0) res_shared().red[i][0][C.warp & 7] = v;
+    if (C.lane == 0) res_shared().own.red[i][C.warp & 7] = v;
 }
 
 /* this thread's rim packets of the block's items, asked for ahead of use */
@@ -194,49 +438,104 @@ __device__ __forceinline__ void rim_ask(const ResCtx &C, unsigned seq, RimAsk &A
         A.lo[x] = 0;
         A.hi[x] = seq;
         if (C.rim_at >= 0 && i < sh.nloc) {
-            const unsigned base = sh.nbr[i][C.rim_nb];
+            const unsigned base = sh.own.nbr[i][C.rim_nb];
             if (base != ~0u)
                 packet_load(rim_at(base + (seq & 1u) * kRim + C.rim_pk), A.lo[x], A.hi[x]);
         }
     }
 }
 
-/* p = z + beta p of the block's items and their halo rings (z of the rims
- * from the plane right after an assembly, else from the packets of exchange
- * `seq`) */
-__device__ __forceinline__ bool fold_p(const ResCtx &C, double beta, bool first, unsigned seq,
-                                       const RimAsk &A)
+/* p = z + beta p of the block's items */
+template <bool SLOW> __device__ __forceinline__ void fold_own(const ResCtx &C, double beta)
 {
     const ResShared &sh = res_shared();
-    const int so = (C.tid / kItemTx + 1) * kPnW + 4 + (C.tid % kItemTx) * kItemVx;
+    const int so = (C.tid / kItemTx + 1) * kPnW + (C.tid % kItemTx) * 2;
     for (int i = C.eng; i < sh.nloc; i += kResEngines) {
-        uint32_t t[16], u[8];
-        tm_ld16(tm_of(C, i) + kTmR, t);
-        tm_ld8(tm_of(C, i) + kTmY, u);
-        double rv[4], dv[4], yv[4], pv[4];
-        unpack4(t, rv);
-        unpack4(t + 8, dv);
-        unpack4(u, yv);
         double *Pn = pn_of(i) + so;
-        lds4(Pn, pv);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) pv[j] = __fma_rn(beta, pv[j], quotient(rv[j], dv[j], yv[j]));
-        reinterpret_cast<double2 *>(Pn)[0] = make_double2(pv[0], pv[1]);
-        reinterpret_cast<double2 *>(Pn)[1] = make_double2(pv[2], pv[3]);
-        __syncwarp();
+        for (int h = 0; h < 2; ++h) {
+            uint32_t t[16];
+            tm_ld16(tm_of(C, i) + h * kTmHalf, t);
+            double rv[2], dv[2], yv[2], pv[2];
+            unpack2(t + 4, rv);
+            unpack2(t + 8, dv);
+            unpack2(t + 12, yv);
+            lds2(Pn + h * kHalf, pv);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                pv[j] = __fma_rn(beta, pv[j],
+                                 SLOW ? __ddiv_rn(rv[j], dv[j]) : quotient(rv[j], dv[j], yv[j]));
+            sts2(Pn + h * kHalf, pv);
+            __syncwarp();
+        }
     }
+}
+__device__ __noinline__ void slow_fold()
+{
+    const ResCtx C = make_ctx();
+    fold_own<true>(C, res_shared().beta);
+}
+
+/* the rim packets of an item: z of its first and last rows and columns */
+__device__ __forceinline__ void send_rims(const ResCtx &C, int i, const double zv[4], unsigned seq)
+{
+    const int ty = C.tid / kItemTx, tx = C.tid % kItemTx;
+    ulonglong2 *rim = rim_at(((blockIdx.x * kResItems + i) * 2 + (seq & 1u)) * kRim);
+    if (ty == 0 || ty == kItemBy - 1) {
+        ulonglong2 *d = rim + (ty == 0 ? 0 : kItemBx) + tx * kItemVx;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) rim_store(d + j, zv[j], seq);
+    }
+    if (tx == 0) rim_store(rim + 2 * kItemBx + ty, zv[0], seq);
+    if (tx == kItemTx - 1) rim_store(rim + 2 * kItemBx + kItemBy + ty, zv[3], seq);
+}
+
+/* z = r / diag, the rims and r.z of the block's items by IEEE divisions */
+__device__ __noinline__ void slow_update(unsigned seq)
+{
+    const ResCtx C = make_ctx();
+    const ResShared &sh = res_shared();
+    for (int i = C.eng; i < sh.nloc; i += kResEngines) {
+        double zv[4], acc = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t t[16];
+            tm_ld16(tm_of(C, i) + h * kTmHalf, t);
+            double rv[2], dv[2];
+            unpack2(t + 4, rv);
+            unpack2(t + 8, dv);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                zv[2 * h + j] = __ddiv_rn(rv[j], dv[j]);
+                acc = __fma_rn(rv[j], zv[2 * h + j], acc);
+            }
+            __syncwarp();
+        }
+        send_rims(C, i, zv, seq);
+        __syncwarp();
+        item_sum(C, i, acc);
+    }
+    __syncthreads();
+}
+
+/* p = z + beta p of the items' halo rings (z from the plane right after an
+ * assembly, else from the packets of exchange `seq`) */
+__device__ __forceinline__ bool fold_rims(const ResCtx &C, double beta, bool first, unsigned seq,
+                                          const RimAsk &A)
+{
+    const ResShared &sh = res_shared();
     bool ok = true;
     if (C.rim_at >= 0) {
 #pragma unroll
         for (int x = 0; x < kResPerEngine; ++x) {
             const int i = x * kResEngines + C.eng;
             if (i >= sh.nloc) continue;
-            const unsigned base = sh.nbr[i][C.rim_nb];
+            const unsigned base = sh.own.nbr[i][C.rim_nb];
             if (base == ~0u) continue;   /* outside the tile: p stays zero */
             double z;
             if (first) {
-                const int li = sh.li[i], gr = (li / sh.T.nbx) * kItemBy - 1 + C.rim_at / kPnW;
-                const int gc = (li % sh.T.nbx) * kItemBx - 4 + C.rim_at % kPnW;
+                const int li = sh.li[i], gr = (li / sh.T.nbx) * kItemBy + C.rim_r;
+                const int gc = (li % sh.T.nbx) * kItemBx + C.rim_c;
                 z = gr < sh.T.nr && gc < sh.T.nc
                         ? ldc((const double *)sh.K.P.z + sh.T.pix + (size_t)gr * sh.T.pitch + gc)
                         : 0.0;
@@ -270,106 +569,131 @@ __device__ __noinline__ bool iterate()
     ResShared &sh = res_shared();
     TileState &S = sh.S;
     const int ty = C.tid / kItemTx, tx = C.tid % kItemTx;
-    const int so = (ty + 1) * kPnW + 4 + tx * kItemVx;
+    const int row = (ty + 1) * kPnW, so = row + tx * 2;
+    /* left neighbour of the first pixel, right neighbour of the last */
+    const int so_l = tx > 0 ? so + kHalf - 1 : row + kLeft;
+    const int so_r = tx < kItemTx - 1 ? so + 2 : row + kRight;
+    const int wo = ty * kWrW + tx * 2, wo_l = tx > 0 ? wo + kHalf - 1 : ty * kWrW + kLeft;
     unsigned seq = sh.seq;
     RimAsk A;
     bool first = true;
     while (true) {
-        if (!fold_p(C, sh.beta, first, seq, A)) return false;
+        if (sh.own.slow) {
+            slow_fold();
+            if (!first) rim_ask(C, seq, A);
+        } else {
+            fold_own<false>(C, sh.beta);
+        }
+        if (!fold_rims(C, sh.beta, first, seq, A)) return false;
         first = false;
         /* q = A p and p.q, in k_solve's order (an arc outside the tile has
          * weight zero and adds nothing) */
-        double q[kResPerEngine][4];
+        /* set to zero: with values left open for items the block does not hold,
+         * the compiler kept all of q in local memory */
+        double q[kResPerEngine][4] = {};
 #pragma unroll
         for (int x = 0; x < kResPerEngine; ++x) {
             const int i = x * kResEngines + C.eng;
             if (i >= sh.nloc) continue;
             const double *Pn = pn_of(i), *WD = wd_of(i), *WR = wr_of(i);
-            double pn[4], up[4], dn[4], wdn[4], wup[4], wrt[4];
-            lds4(Pn + so, pn);
-            lds4(Pn + so - kPnW, up);
-            lds4(Pn + so + kPnW, dn);
-            lds4(WD + (ty + 1) * kItemBx + tx * kItemVx, wdn);
-            lds4(WD + ty * kItemBx + tx * kItemVx, wup);
-            lds4(WR + ty * kWrW2 + 4 + tx * kItemVx, wrt);
-            const double lf = Pn[so - 1], rt = Pn[so + 4], wlf = WR[ty * kWrW2 + 3 + tx * kItemVx];
-            double acc = 0.0;
+            double acc = 0.0, xl = Pn[so_l], wl = WR[wo_l];   /* left pixel and arc */
+            double pn[2], nx[2];
+            lds2(Pn + so, pn);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const double xa = pn[j];
-                const double xl = j == 0 ? lf : pn[j - 1], xr = j == 3 ? rt : pn[j + 1];
-                double y = (double)kLapEpsF * xa;
-                y = __fma_rn(wdn[j], xa - dn[j], y);
-                y = __fma_rn(wup[j], xa - up[j], y);
-                y = __fma_rn(wrt[j], xa - xr, y);
-                y = __fma_rn(j == 0 ? wlf : wrt[j - 1], xa - xl, y);
-                q[x][j] = y;
-                acc = __fma_rn(xa, y, acc);
+            for (int h = 0; h < 2; ++h) {
+                double up[2], dn[2], wdn[2], wup[2], wrt[2];
+                if (h == 0) lds2(Pn + so + kHalf, nx);
+                else nx[0] = Pn[so_r];
+                lds2(Pn + so - kPnW + h * kHalf, up);
+                lds2(Pn + so + kPnW + h * kHalf, dn);
+                lds2(WD + (ty + 1) * kItemBx + tx * 2 + h * kHalf, wdn);
+                lds2(WD + ty * kItemBx + tx * 2 + h * kHalf, wup);
+                lds2(WR + wo + h * kHalf, wrt);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const double xa = pn[j], xr = j == 0 ? pn[1] : nx[0];
+                    double y = (double)kLapEpsF * xa;
+                    y = __fma_rn(wdn[j], xa - dn[j], y);
+                    y = __fma_rn(wup[j], xa - up[j], y);
+                    y = __fma_rn(wrt[j], xa - xr, y);
+                    y = __fma_rn(wl, xa - xl, y);
+                    q[x][2 * h + j] = y;
+                    acc = __fma_rn(xa, y, acc);
+                    xl = xa;
+                    wl = wrt[j];
+                }
+                pn[0] = nx[0];
+                pn[1] = nx[1];
             }
             item_sum(C, i, acc);
         }
         __syncthreads();
-        block_partials(C, 1);
-        send_partials(C, 1, ++seq);
-        double tot[1];
-        if (!totals<1>(C, seq, tot)) return false;
+        block_partial(C);
+        send_partial(++seq);
+        double tot;
+        if (!total(C, seq, tot)) return false;
         if (threadIdx.x == 0) {
-            if (tot[0] <= 0.0) sh.active = 0;
-            else sh.alpha = S.rz / tot[0];
+            if (tot <= 0.0) sh.active = 0;
+            else sh.alpha = quotient_pos(S.rz, tot);
         }
         __syncthreads();
         if (!sh.active) break;
         /* x += alpha p, r -= alpha q, z = r / diag, r.z; the rims' z */
         const double alpha = sh.alpha;
+        bool odd = false;
         ++seq;
 #pragma unroll
         for (int x = 0; x < kResPerEngine; ++x) {
             const int i = x * kResEngines + C.eng;
             if (i >= sh.nloc) continue;
-            uint32_t t[16], u[16];
-            tm_ld16(tm_of(C, i) + kTmX, t);
-            tm_ld16(tm_of(C, i) + kTmD, u);
-            double xv[4], rv[4], dv[4], yv[4], pv[4], zv[4], acc = 0.0;
-            unpack4(t, xv);
-            unpack4(t + 8, rv);
-            unpack4(u, dv);
-            unpack4(u + 8, yv);
-            lds4(pn_of(i) + so, pv);
+            double zv[4], acc = 0.0;
+            bool mine = false;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                xv[j] = __fma_rn(alpha, pv[j], xv[j]);
-                rv[j] = __fma_rn(-alpha, q[x][j], rv[j]);
-                zv[j] = quotient(rv[j], dv[j], yv[j]);
-                acc = __fma_rn(rv[j], zv[j], acc);
-            }
-            __syncwarp();
-            tm_st4d(tm_of(C, i) + kTmX, xv);
-            tm_st4d(tm_of(C, i) + kTmR, rv);
-            ulonglong2 *rim = rim_at(((blockIdx.x * kResItems + i) * 2 + (seq & 1u)) * kRim);
-            if (ty == 0 || ty == kItemBy - 1) {
-                ulonglong2 *d = rim + (ty == 0 ? 0 : kItemBx) + tx * kItemVx;
+            for (int h = 0; h < 2; ++h) {
+                uint32_t t[16];
+                tm_ld16(tm_of(C, i) + h * kTmHalf, t);
+                double xv[2], rv[2], dv[2], yv[2], pv[2];
+                unpack2(t, xv);
+                unpack2(t + 4, rv);
+                unpack2(t + 8, dv);
+                unpack2(t + 12, yv);
+                lds2(pn_of(i) + so + h * kHalf, pv);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) rim_store(d + j, zv[j], seq);
+                for (int j = 0; j < 2; ++j) {
+                    xv[j] = __fma_rn(alpha, pv[j], xv[j]);
+                    rv[j] = __fma_rn(-alpha, q[x][2 * h + j], rv[j]);
+                    mine = mine || __double2hiint(yv[j]) == 0 || res_odd(rv[j]);
+                    const double z = quotient(rv[j], dv[j], yv[j]);
+                    zv[2 * h + j] = z;
+                    acc = __fma_rn(rv[j], z, acc);
+                }
+                float f[8];
+                pack2(xv, f);
+                pack2(rv, f + 4);
+                __syncwarp();
+                tm_st8(tm_of(C, i) + h * kTmHalf, f);
             }
-            if (tx == 0) rim_store(rim + 2 * kItemBx + ty, zv[0], seq);
-            if (tx == kItemTx - 1) rim_store(rim + 2 * kItemBx + kItemBy + ty, zv[3], seq);
+            odd = odd || mine;
+            if (!mine) send_rims(C, i, zv, seq);   /* else slow_update does */
             __syncwarp();
             item_sum(C, i, acc);
         }
         tm_wait_st();
-        __syncthreads();
-        block_partials(C, 1);
-        send_partials(C, 1, seq);
+        odd = __syncthreads_or(odd);
+        if (odd) slow_update(seq);
+        if (threadIdx.x == 0) sh.own.slow = odd;
+        block_partial(C);
+        send_partial(seq);
         rim_ask(C, seq, A);
-        if (!totals<1>(C, seq, tot)) return false;
+        if (!total(C, seq, tot)) return false;
         if (threadIdx.x == 0) {
             const int it = S.iter + 1;
             S.iter = it;
-            if (tot[0] < S.thr || it >= sh.K.sp.max_iter) {
+            if (tot < S.thr || it >= sh.K.sp.max_iter) {
                 sh.active = 0;
             } else {
-                sh.beta = tot[0] / S.rz;
-                S.rz = tot[0];
+                sh.beta = quotient_pos(tot, S.rz);
+                S.rz = tot;
             }
             if ((it & 63) == 63 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
         }
@@ -394,9 +718,9 @@ template <bool WLS> __device__ __noinline__ bool assemble(bool zero_x, double &r
     }
     __syncthreads();
     const unsigned seq = sh.seq + 1;
-    block_partials(C, 1);
-    send_partials(C, 1, seq);
-    if (!totals<1>(C, seq, &rz)) return false;
+    block_partial(C);
+    send_partial(seq);
+    if (!total(C, seq, rz)) return false;
     if (threadIdx.x == 0) sh.seq = seq;
     return group_sync();
 }
@@ -449,7 +773,14 @@ template <bool WLS> __device__ __forceinline__ bool run_tile()
 template <bool WLS>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident64(const __grid_constant__ ResParams K)
 {
-    resident_blocks(K, [] { return run_tile<WLS>(); });
+    resident_blocks(
+        K,
+        [](const ResTile &R) {
+            ResShared &sh = res_shared();
+            sh.own.g = R.g;
+            sh.nloc = res_count(sh.T.nitems, sh.member, R.g);
+        },
+        [] { return run_tile<WLS>(); });
 }
 
 }  // namespace

@@ -8,53 +8,96 @@
 #include <cmath>
 
 namespace cuphu {
+namespace {
 
-/* most items any block of a group of 2^g holds */
-static int res_most(int nitems, int g)
+/* how a tile may be split: members (with items: nact) and the most items of
+ * one of them */
+struct Shape {
+    int g = 0, a = 0, b = 0, rcols = 0;
+    int nmem = 0, nact = 0, most = 0;
+    bool ok() const { return nact > 0; }
+};
+
+/* FP64: the smallest group of 2^g members that keeps to k items per block */
+Shape slots_shape(int nitems, int k, int nblk)
 {
-    int most = 0;
-    for (int m = 0; m < (1 << g); ++m) most = std::max(most, res_count(nitems, m, g));
-    return most;
+    Shape s;
+    for (int g = 3; g <= kResMaxG; ++g) {
+        int most = 0, nact = 0;
+        for (int m = 0; m < (1 << g); ++m) {
+            const int n = res_count(nitems, m, g);
+            most = std::max(most, n);
+            nact += n > 0;
+        }
+        if (most > k || nact > nblk) continue;
+        s.g = g;
+        s.nmem = 1 << g;
+        s.nact = nact;
+        s.most = most;
+        break;
+    }
+    return s;
 }
 
-/* Choose the group sizes and the schedule.  An iteration of a tile costs about
- * c0 + c1 x (most items of one block): c0 the exchange, c1 one item (both
- * measured, in us).  Small groups spread the exchange over more work per block
- * and let many tiles run side by side; large ones shorten a tile's
- * iteration.  The bound k on the items of a block that gives the smallest
- * estimated makespan over the job's tiles is taken.  Tiles that no group holds
- * (above 1792 items in mixed precision, 1024 in FP64) are streamed. */
+/* mixed: the region of at most k items that needs the fewest blocks, then the
+ * one with the shortest rim */
+Shape region_shape(const TileDesc &T, int k, int nblk)
+{
+    const int nby = T.nitems / T.nbx;
+    Shape s;
+    int best_rim = 0;
+    for (int b = 1; b <= kResMaxB && b <= T.nbx; ++b)
+        for (int a = 1; a * b <= k && a <= nby; ++a) {
+            const int rrows = (nby + a - 1) / a, rcols = (T.nbx + b - 1) / b, n = rrows * rcols;
+            if (n > std::min(nblk, kResMaxBlocks)) continue;
+            const int rim = 16 * a + 64 * b;
+            if (s.ok() && (n > s.nact || (n == s.nact && rim >= best_rim))) continue;
+            s.a = a;
+            s.b = b;
+            s.rcols = rcols;
+            s.nmem = s.nact = n;
+            s.most = a * b;
+            best_rim = rim;
+        }
+    return s;
+}
+}  // namespace
+
+/* Choose the splits and the schedule.  An iteration of a tile costs about c0 +
+ * c1 x (most items of one block): c0 the exchanges, c1 one item (measured, in
+ * us).  Small groups spread the exchange over more work per block and let many
+ * tiles run side by side; large ones shorten a tile's iteration.  The bound k
+ * on the items of a block that gives the smallest estimated makespan over the
+ * job's tiles is taken.  Tiles that no group holds (above 16 items for each
+ * of the GPU's SMs in mixed precision, 1024 items in FP64) are streamed. */
 void plan_resident(const std::vector<TileDesc> &tiles, int nblk, bool fp64, ResidentPlan &R)
 {
     const int cap = fp64 ? kResItems64 : kResItemsMixed;
-    const double c0 = fp64 ? 5.0 : 3.8, c1 = 0.6;
+    const double c0 = fp64 ? 7.0 : 3.3, c1 = fp64 ? 0.9 : 0.42;
     R = ResidentPlan();
+    /* the split of tile t under the bound k, or the nearest one above it */
+    auto shape = [&](int t, int k) {
+        Shape s;
+        for (; k <= cap && !s.ok(); ++k)
+            s = fp64 ? slots_shape(tiles[t].nitems, k, nblk) : region_shape(tiles[t], k, nblk);
+        return s;
+    };
+    auto cost = [&](int t, const Shape &s) {
+        return std::sqrt((double)tiles[t].nitems) * (c0 + c1 * s.most);
+    };
     std::vector<int> fit;
     for (int t = 0; t < (int)tiles.size(); ++t)
-        if (res_most(tiles[t].nitems, kResMaxG) <= cap && nblk >= (1 << kResMaxG)) fit.push_back(t);
+        if (shape(t, cap).ok()) fit.push_back(t);
         else R.streamed.push_back(t);
     if (fit.empty()) return;
-    auto shape = [&](int nitems, int k, int &g, int &most) {
-        for (g = 3; g < kResMaxG; ++g)
-            if ((most = res_most(nitems, g)) <= k) return;
-        most = res_most(nitems, g);
-    };
-    auto active = [&](int nitems, int g) {
-        int a = 0;
-        for (int m = 0; m < (1 << g); ++m) a += res_count(nitems, m, g) > 0;
-        return a;
-    };
     int best_k = cap;
     double best = 0.0;
     for (int k = 1; k <= cap; ++k) {
         double area = 0.0, longest = 0.0;
         for (int t : fit) {
-            int g, most;
-            shape(tiles[t].nitems, k, g, most);
-            const int a = active(tiles[t].nitems, g);
-            const double d = std::sqrt((double)tiles[t].nitems) * (c0 + c1 * most);
-            /* groups that do not pack waste the blocks left over */
-            area += d / (nblk / a);
+            const Shape s = shape(t, k);
+            const double d = cost(t, s);
+            area += d / (nblk / s.nact);   /* groups that do not pack waste what is left over */
             longest = std::max(longest, d);
         }
         const double est = std::max(area, longest);
@@ -63,13 +106,11 @@ void plan_resident(const std::vector<TileDesc> &tiles, int nblk, bool fp64, Resi
             best_k = k;
         }
     }
-    struct Job { int t, g, a; double d; };
+    struct Job { int t; Shape s; double d; };
     std::vector<Job> jobs;
     for (int t : fit) {
-        int g, most;
-        shape(tiles[t].nitems, best_k, g, most);
-        jobs.push_back({t, g, active(tiles[t].nitems, g),
-                        std::sqrt((double)tiles[t].nitems) * (c0 + c1 * most)});
+        const Shape s = shape(t, best_k);
+        jobs.push_back({t, s, cost(t, s)});
     }
     std::stable_sort(jobs.begin(), jobs.end(), [](const Job &a, const Job &b) { return a.d > b.d; });
     /* longest first onto the blocks that are free first; blocks process
@@ -81,12 +122,13 @@ void plan_resident(const std::vector<TileDesc> &tiles, int nblk, bool fp64, Resi
     for (const Job &j : jobs) {
         for (int b = 0; b < nblk; ++b) idx[b] = b;
         std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return load[a] < load[b]; });
-        const double start = load[idx[j.a - 1]];
+        const double start = load[idx[j.s.nact - 1]];
         const int sched = (int)R.sched.size();
-        R.sched.push_back({j.t, j.g, j.a, (int)R.phys.size()});
+        R.sched.push_back({j.t, j.s.nmem, j.s.nact, (int)R.phys.size(), j.s.g, j.s.a, j.s.b,
+                           j.s.rcols});
         int used = 0;
-        for (int m = 0; m < (1 << j.g); ++m) {
-            if (res_count(tiles[j.t].nitems, m, j.g) == 0) {
+        for (int m = 0; m < j.s.nmem; ++m) {
+            if (fp64 && res_count(tiles[j.t].nitems, m, j.s.g) == 0) {
                 R.phys.push_back(0xffff);
                 continue;
             }
@@ -106,15 +148,16 @@ void plan_resident(const std::vector<TileDesc> &tiles, int nblk, bool fp64, Resi
     while (R.nblk > 1 && per[R.nblk - 1].empty()) --R.nblk;
 }
 
-constexpr size_t kRimPx = 2 * kItemBx + 2 * kItemBy;   /* rim packets of an item, per buffer */
+/* rim packets: FP64 16 bytes for the ring of each item, mixed 8 bytes for the
+ * four sides of a region (256 pixels each), two buffers */
 size_t resident_rim_bytes(int nblk, bool fp64)
 {
-    return fp64 ? (size_t)nblk * kResItems64 * 2 * kRimPx * 16
-                : (size_t)nblk * kResItemsMixed * 2 * kRimPx * 8;
+    return fp64 ? (size_t)nblk * kResItems64 * 2 * (2 * kItemBx + 2 * kItemBy) * 16
+                : (size_t)nblk * 2 * 4 * 256 * 8;
 }
-size_t resident_mail_bytes(int nblk)
+size_t resident_mail_bytes(int nblk, bool fp64)
 {
-    return (size_t)nblk * 2 * kNComp * kResMembers * sizeof(ulonglong2);
+    return (size_t)nblk * 2 * (fp64 ? 4 * kResMembers : kNComp * kResMaxBlocks) * sizeof(ulonglong2);
 }
 
 }  // namespace cuphu

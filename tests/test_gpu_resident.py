@@ -42,8 +42,8 @@ def scene(nr, nc, seed, blocked=False):
 @pytest.mark.parametrize("shape,blocked", [
     ((1, 1), False), ((1, 70), False), ((70, 1), False), ((2, 64), False), ((16, 64), True),
     ((17, 65), False), ((15, 1037), True), ((1025, 63), False), ((255, 1030), False),
-    ((512, 512), True), ((967, 961), False), ((1000, 1102), True), ((1344, 1340), False),
-    ((1424, 1409), False)])
+    ((512, 512), True), ((967, 961), False), ((1000, 1102), True), ((270, 1030), True),
+    ((1536, 1536), False), ((1540, 1537), False)])
 def test_on_chip_solve_matches_fp64(torch_cuda, shape, blocked):
     costs, ph = scene(*shape, seed=shape[0] + 3 * shape[1], blocked=blocked)
     _, k64, c64, s64 = gpu_solve(torch_cuda, costs, ph, precision=1, n_irls=2)
