@@ -21,6 +21,7 @@
  */
 #include "kernels.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -42,7 +43,11 @@ struct PhaseStaging {
 
 PhaseStaging g_stage[64];
 
-constexpr size_t kChunk = (size_t)1 << 20;   /* pixels per upload */
+/* Pixels of a chunk: a chunk is one thread's unit of work and one upload.
+ * About four per thread, at least 2^14 (0.3 ms of atan2f, several times the
+ * start of a thread) and at most 2^20.  One size of 2^20 left scenes below
+ * 1 Mpx to a single thread: 5.3 of the 28 ms of a 512x512 call. */
+constexpr size_t kMinChunk = (size_t)1 << 14, kMaxChunk = (size_t)1 << 20;
 
 /* one sample: non-finite samples read as 0 (cuphu.unwrap replaces them,
  * _unwrap.py:515-520); host float atan2, shift, device re-wrap */
@@ -79,9 +84,15 @@ int host_threads()
 
 }  // namespace
 
+static size_t chunk_of(size_t n)
+{
+    const size_t c = n / (4 * (size_t)host_threads()) + 1;
+    return std::min(std::max(c, kMinChunk), kMaxChunk);
+}
+
 void compute_host_phase(const float *c64, const float *re, const float *im, size_t n, float *out)
 {
-    const size_t nch = (n + kChunk - 1) / kChunk;
+    const size_t chunk = chunk_of(n), nch = (n + chunk - 1) / chunk;
     const int nth = (int)std::min<size_t>((size_t)host_threads(), nch);
     if (nth <= 1) {
         phase_range(c64, re, im, out, 0, n);
@@ -95,7 +106,7 @@ void compute_host_phase(const float *c64, const float *re, const float *im, size
             for (;;) {
                 size_t c = next.fetch_add(1, std::memory_order_relaxed);
                 if (c >= nch) return;
-                phase_range(c64, re, im, out, c * kChunk, std::min(n, (c + 1) * kChunk));
+                phase_range(c64, re, im, out, c * chunk, std::min(n, (c + 1) * chunk));
             }
         });
     for (auto &th : pool) th.join();
@@ -128,7 +139,7 @@ int upload_host_phase(const float *c64, const float *re, const float *im, size_t
         P.buf = b;
         P.cap = n;
     }
-    const size_t nch = (n + kChunk - 1) / kChunk;
+    const size_t chunk = chunk_of(n), nch = (n + chunk - 1) / chunk;
     const int nth = (int)std::min<size_t>((size_t)host_threads(), nch);
     int rc = 0;
     if (nth <= 1) {
@@ -146,7 +157,7 @@ int upload_host_phase(const float *c64, const float *re, const float *im, size_t
                 for (;;) {
                     size_t c = next.fetch_add(1, std::memory_order_relaxed);
                     if (c >= nch) return;
-                    size_t a = c * kChunk, b = std::min(n, a + kChunk);
+                    size_t a = c * chunk, b = std::min(n, a + chunk);
                     phase_range(c64, re, im, P.buf, a, b);
                     ready[c].store(1, std::memory_order_release);
                 }
@@ -154,7 +165,7 @@ int upload_host_phase(const float *c64, const float *re, const float *im, size_t
         for (size_t c = 0; c < nch; ++c) {
             while (!ready[c].load(std::memory_order_acquire)) std::this_thread::yield();
             if (rc) continue;
-            size_t a = c * kChunk, len = std::min(n, a + kChunk) - a;
+            size_t a = c * chunk, len = std::min(n, a + chunk) - a;
             rc = cuda_fail(cudaMemcpyAsync(d_ph + a, P.buf + a, len * sizeof(float),
                                            cudaMemcpyHostToDevice, s),
                            "H2D phase");
