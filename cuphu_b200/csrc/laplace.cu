@@ -112,24 +112,6 @@ __device__ __forceinline__ void item_partials(const TileDesc &T, int a, int b, d
     }
 }
 
-/* block tree without the leading barrier, for item loops: consecutive items
- * pass alternating halves of the scratch (sw, sw + 8), so a warp that runs
- * ahead into the next item never overwrites warp sums that warp 0 has not
- * read; returns after the barrier that follows the warp sums, so every thread
- * has finished the caller's work on the item */
-__device__ __forceinline__ double block_sum_item(double v, double *sw)
-{
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) sw[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? sw[lane] : 0.0;
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    }
-    return v;
-}
-
 /* A block has written the partials of its items [a, b) of tile t for this
  * phase (thread 0 writes every partial of a block).  The block whose items
  * complete the tile's count computes the canonical tile total once and
@@ -308,8 +290,8 @@ template <typename V> __host__ __device__ constexpr size_t pn_bytes()
 /* NS: stages of the shared-memory ring (items in flight per block) */
 template <typename V, int NS> __host__ __device__ constexpr size_t solve_smem_bytes()
 {
-    /* mixed mode double-buffers Pn by item parity */
-    return NS * stage_bytes<V>() + (sizeof(V) == 4 ? 2 : 1) * pn_bytes<V>() + 128;
+    /* Pn is double-buffered by item parity */
+    return NS * stage_bytes<V>() + 2 * pn_bytes<V>() + 128;
 }
 
 
@@ -406,25 +388,23 @@ __device__ __forceinline__ void sld4(const double *p, double v[4])
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
-/* stencil pass on a staged item (FP64, the oracle's operation order):
- * p_new = z + beta p_old (own + halo ring), q = A p_new, thread partial of
- * p.q */
-__device__ double compute_a(const TileDesc &T, int li, const SolverPlanes &P, double *pnew_all,
-                            bool first, double beta, const char *stage, double *Pn)
+/* stencil pass on a staged item (FP64, the oracle's operation order), in two
+ * halves around the item's barrier.  a1: p_new = z + beta p_old of the own
+ * pixels and the halo ring into Pn.  a2: q = A p_new; returns the thread's
+ * partial of p.q. */
+__device__ __forceinline__ void compute_a1(const TileDesc &T, int li, bool first, double beta,
+                                           const char *stage, double *Pn)
 {
     const int r0b = (li / T.nbx) * kItemBy, c0b = (li % T.nbx) * kItemBx;
     const double *Z = (const double *)stage;
     const double *PO = (const double *)(stage + StageA::kVec);
-    const float *WD = (const float *)(stage + 2 * StageA::kVec);
-    const float *WR = (const float *)(stage + 2 * StageA::kVec + StageA::kWd);
     const int nr = T.nr, nc = T.nc;
     const int ty = threadIdx.x / kItemTx, tx = threadIdx.x % kItemTx;
     const int r = r0b + ty, c0 = c0b + tx * kItemVx;
-    const bool own = r < nr && c0 < nc;
     /* own p_new: row ty+1, columns 4 + 4 tx .. +3 */
     double pn[4] = {0.0, 0.0, 0.0, 0.0};
     const int so = (ty + 1) * kSegW + 4 + tx * kItemVx;
-    if (own) {
+    if (r < nr && c0 < nc) {
         double zv[4], pv[4] = {0.0, 0.0, 0.0, 0.0};
         sld4(Z + so, zv);
         if (!first) sld4(PO + so, pv);
@@ -432,8 +412,8 @@ __device__ double compute_a(const TileDesc &T, int li, const SolverPlanes &P, do
         for (int j = 0; j < kItemVx; ++j)
             if (c0 + j < nc) pn[j] = first ? zv[j] : __fma_rn(beta, pv[j], zv[j]);
     }
-#pragma unroll
-    for (int j = 0; j < kItemVx; ++j) Pn[so + j] = pn[j];
+    reinterpret_cast<double2 *>(Pn + so)[0] = make_double2(pn[0], pn[1]);
+    reinterpret_cast<double2 *>(Pn + so)[1] = make_double2(pn[2], pn[3]);
     /* halo ring: rows above/below (64 each), columns left/right (16 each) */
     if (threadIdx.x < 2 * kItemBx + 2 * kItemBy) {
         int h = threadIdx.x, i, jc;
@@ -449,38 +429,49 @@ __device__ double compute_a(const TileDesc &T, int li, const SolverPlanes &P, do
         }
         Pn[i * kSegW + jc] = v;
     }
-    __syncthreads();
+}
+
+__device__ __forceinline__ double compute_a2(const TileDesc &T, int li, const SolverPlanes &P,
+                                             double *pnew_all, const char *stage, const double *Pn)
+{
+    const int r0b = (li / T.nbx) * kItemBy, c0b = (li % T.nbx) * kItemBx;
+    const float *WD = (const float *)(stage + 2 * StageA::kVec);
+    const float *WR = (const float *)(stage + 2 * StageA::kVec + StageA::kWd);
+    const int nr = T.nr, nc = T.nc;
+    const int ty = threadIdx.x / kItemTx, tx = threadIdx.x % kItemTx;
+    const int r = r0b + ty, c0 = c0b + tx * kItemVx;
+    if (r >= nr || c0 >= nc) return 0.0;
+    const int so = (ty + 1) * kSegW + 4 + tx * kItemVx;
     double acc = 0.0;
-    if (own) {
-        double up[4], dn[4], qv[4] = {0.0, 0.0, 0.0, 0.0};
-        float wdn[4], wup[4], wrt[4];
-        sld4(Pn + so - kSegW, up);
-        sld4(Pn + so + kSegW, dn);
-        double lf = Pn[so - 1], rt = Pn[so + 4];
-        sld4(WD + (ty + 1) * kItemBx + tx * kItemVx, wdn);
-        sld4(WD + ty * kItemBx + tx * kItemVx, wup);
-        sld4(WR + ty * kWrW + tx * kItemVx + 4, wrt);
-        float wlf = WR[ty * kWrW + tx * kItemVx + 3];
+    double pn[4], up[4], dn[4], qv[4] = {0.0, 0.0, 0.0, 0.0};
+    float wdn[4], wup[4], wrt[4];
+    sld4(Pn + so, pn);
+    sld4(Pn + so - kSegW, up);
+    sld4(Pn + so + kSegW, dn);
+    double lf = Pn[so - 1], rt = Pn[so + 4];
+    sld4(WD + (ty + 1) * kItemBx + tx * kItemVx, wdn);
+    sld4(WD + ty * kItemBx + tx * kItemVx, wup);
+    sld4(WR + ty * kWrW + tx * kItemVx + 4, wrt);
+    float wlf = WR[ty * kWrW + tx * kItemVx + 3];
 #pragma unroll
-        for (int j = 0; j < kItemVx; ++j) {
-            int c = c0 + j;
-            if (c >= nc) continue;
-            double xl = j == 0 ? lf : pn[j - 1];
-            double xr = j == kItemVx - 1 ? rt : pn[j + 1];
-            float wl = j == 0 ? wlf : wrt[j - 1];
-            double xa = pn[j];
-            double y = (double)kLapEpsF * xa;
-            if (r < nr - 1) y = __fma_rn((double)wdn[j], xa - dn[j], y);
-            if (r > 0)      y = __fma_rn((double)wup[j], xa - up[j], y);
-            if (c < nc - 1) y = __fma_rn((double)wrt[j], xa - xr, y);
-            if (c > 0)      y = __fma_rn((double)wl, xa - xl, y);
-            qv[j] = y;
-            acc = __fma_rn(pn[j], y, acc);
-        }
-        size_t o = T.pix + (size_t)r * T.pitch + c0;
-        st4(pnew_all + o, pn);
-        st4((double *)P.q + o, qv);
+    for (int j = 0; j < kItemVx; ++j) {
+        int c = c0 + j;
+        if (c >= nc) continue;
+        double xl = j == 0 ? lf : pn[j - 1];
+        double xr = j == kItemVx - 1 ? rt : pn[j + 1];
+        float wl = j == 0 ? wlf : wrt[j - 1];
+        double xa = pn[j];
+        double y = (double)kLapEpsF * xa;
+        if (r < nr - 1) y = __fma_rn((double)wdn[j], xa - dn[j], y);
+        if (r > 0)      y = __fma_rn((double)wup[j], xa - up[j], y);
+        if (c < nc - 1) y = __fma_rn((double)wrt[j], xa - xr, y);
+        if (c > 0)      y = __fma_rn((double)wl, xa - xl, y);
+        qv[j] = y;
+        acc = __fma_rn(pn[j], y, acc);
     }
+    size_t o = T.pix + (size_t)r * T.pitch + c0;
+    st4(pnew_all + o, pn);
+    st4((double *)P.q + o, qv);
     return acc;
 }
 
@@ -505,7 +496,7 @@ __device__ __forceinline__ void issue_b(const TileDesc &T, int li, const SolveMa
 }
 
 /* update pass (FP64): x += alpha p; r -= alpha q; z = r / diag; partial r.z */
-__device__ double compute_b(const TileDesc &T, int li, const SolverPlanes &P, double alpha,
+__device__ __forceinline__ double compute_b(const TileDesc &T, int li, const SolverPlanes &P, double alpha,
                             bool update_r, const char *stage)
 {
     const int r0b = (li / T.nbx) * kItemBy, c0b = (li % T.nbx) * kItemBx;
@@ -998,73 +989,6 @@ __device__ __forceinline__ Cursor cursor_next(Cursor c, const SliceCtl &sc, cons
     return cursor_active(Cursor{rev ? c.p - 1 : c.p + 1, c.t}, sc, g, st, ntiles, rev);
 }
 
-/* run a staged FP64 pass over this block's slice.  KIND 0: the stencil
- * pass, KIND 1: the update pass.  NS items are in flight; the stage of
- * item k is refilled with item k+NS right after the barrier of item k's
- * reduction, which every thread reaches only after its last read of the
- * stage and Pn. */
-template <int KIND, int NS>
-__device__ void run_pass(const SliceCtl &sc, const TileDesc *gt, const TileState *st, int ntiles,
-                         const SolverPlanes &P, const SolveMaps &M, int psel, double *pvec,
-                         bool flag, double *part, double *tot, unsigned *cnt, double *sw,
-                         double *s_bcast, int *s_flag, double *Pn, char *stages, uint64_t *bars,
-                         uint32_t &parity, SolverCtl *ctl, long long timeout_ns, bool rev)
-{
-    constexpr size_t SB = stage_bytes<double>();
-    const bool red = KIND == 0 || flag;
-    if (sc.s0 >= sc.s1) return;
-    Cursor ci = cursor_first(sc, gt, st, ntiles, rev);
-    if (!cursor_live(ci, sc)) return;
-    Cursor cc = ci;
-    if (threadIdx.x == 0) {
-        fence_async_global();
-        fence_async_smem();
-    }
-    for (int k = 0; k < NS && cursor_live(ci, sc); ++k) {
-        if (threadIdx.x == 0) {
-            const TileDesc &T = stile(sc, gt, ci.t);
-            int li = ci.p - sc.pre[ci.t];
-            if (KIND == 0) issue_a(T, li, M, psel, flag, stages + k * SB, bars + k);
-            else issue_b(T, li, M, psel, flag, stages + k * SB, bars + k);
-        }
-        ci = cursor_next(ci, sc, gt, st, ntiles, rev);
-    }
-    int done = 0;
-    while (cursor_live(cc, sc)) {
-        int s = done % NS;
-        mbar_wait(bars + s, (parity >> s) & 1u, ctl, timeout_ns);
-        parity ^= 1u << s;
-        ++done;
-        const TileDesc &T = stile(sc, gt, cc.t);
-        int li = cc.p - sc.pre[cc.t];
-        double acc;
-        if (KIND == 0)
-            acc = compute_a(T, li, P, pvec, flag, sbeta(sc, st, cc.t), stages + s * SB, Pn);
-        else
-            acc = compute_b(T, li, P, salpha(sc, st, cc.t), flag, stages + s * SB);
-        double bs = block_sum_item(acc, sw + 8 * (done & 1));   /* contains the item barrier */
-        if (threadIdx.x == 0) {
-            if (red) part[T.item0 + li] = bs;
-            if (cursor_live(ci, sc)) {
-                fence_async_smem();
-                const TileDesc &Tn = stile(sc, gt, ci.t);
-                int ln = ci.p - sc.pre[ci.t];
-                if (KIND == 0) issue_a(Tn, ln, M, psel, flag, stages + s * SB, bars + s);
-                else issue_b(Tn, ln, M, psel, flag, stages + s * SB, bars + s);
-            }
-        }
-        if (cursor_live(ci, sc)) ci = cursor_next(ci, sc, gt, st, ntiles, rev);
-        Cursor nx = cursor_next(cc, sc, gt, st, ntiles, rev);
-        if (red && (!cursor_live(nx, sc) || nx.t != cc.t)) {
-            int a, b;
-            slice_items(sc, T, cc.t, a, b);
-            seg_done(T, cc.t, b - a, part, tot, cnt, sw, s_bcast, s_flag);
-        }
-        cc = nx;
-    }
-    __syncthreads();
-}
-
 /* The mixed pass over this block's slice, staged like run_pass but with one
  * block barrier per item.  Pn and the warp partials alternate between two
  * buffers by item parity.  After the barrier of item k (between its two
@@ -1083,6 +1007,106 @@ __device__ __forceinline__ void store_item_comp(const double (*red)[8], int c, d
     for (int off = kItemThreads / 64; off > 0; off >>= 1)
         x += __shfl_down_sync(0xffffffffu, x, off);
     if (lane == 0) part[(size_t)c * nitems + item] = x;
+}
+
+/* Run a staged FP64 pass over this block's slice.  KIND 0: the stencil pass,
+ * KIND 1: the update pass.  NS items are in flight and an item costs one
+ * block barrier.  Update pass: all threads have read item k's stage at its
+ * barrier, so the stage is refilled with item k+NS right there, by warp 7,
+ * while warp 0 forms the item's partial and the others go on.  Stencil pass:
+ * the barrier lies between the item's halves (p_new is complete), every
+ * thread has finished item k-1 there, so that item's stage is refilled and
+ * its partial formed.  Pn and the warp sums alternate between two buffers.
+ * (With the partial's two trees between the last read of a stage and its
+ * refill, and two barriers per item, a 2048^2 iteration took 125 us, now
+ * 119.) */
+template <int KIND, int NS>
+__device__ void run_pass(const SliceCtl &sc, const TileDesc *gt, const TileState *st, int ntiles,
+                         const SolverPlanes &P, const SolveMaps &M, int psel, double *pvec,
+                         bool flag, double *part, double *tot, unsigned *cnt, double *sw,
+                         double (*red)[kNComp][8], double *s_bcast, int *s_flag, double *Pn2,
+                         char *stages, uint64_t *bars, uint32_t &parity, SolverCtl *ctl,
+                         long long timeout_ns, bool rev)
+{
+    constexpr size_t SB = stage_bytes<double>();
+    constexpr size_t PNE = pn_bytes<double>() / sizeof(double);
+    const bool sums = KIND == 0 || flag;
+    if (sc.s0 >= sc.s1) return;
+    Cursor ci = cursor_first(sc, gt, st, ntiles, rev);
+    if (!cursor_live(ci, sc)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool issuer = threadIdx.x == kItemThreads - 32;
+    Cursor cc = ci;
+    auto issue = [&](int s) {
+        const TileDesc &T = stile(sc, gt, ci.t);
+        const int li = ci.p - sc.pre[ci.t];
+        if (KIND == 0) issue_a(T, li, M, psel, flag, stages + s * SB, bars + s);
+        else issue_b(T, li, M, psel, flag, stages + s * SB, bars + s);
+    };
+    if (issuer) {
+        fence_async_global();
+        fence_async_smem();
+    }
+    for (int k = 0; k < NS && cursor_live(ci, sc); ++k) {
+        if (issuer) issue(k);
+        ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+    }
+    int k = 0, prev = -1;   /* item number in the pass; item k-1 (stencil pass) */
+    while (cursor_live(cc, sc)) {
+        const int s = k % NS;
+        mbar_wait(bars + s, (parity >> s) & 1u, ctl, timeout_ns);
+        parity ^= 1u << s;
+        const TileDesc &T = stile(sc, gt, cc.t);
+        const int li = cc.p - sc.pre[cc.t];
+        double acc;
+        if (KIND == 0) {
+            double *Pn = Pn2 + (k & 1) * PNE;
+            compute_a1(T, li, flag, sbeta(sc, st, cc.t), stages + s * SB, Pn);
+            __syncthreads();
+            if (prev >= 0) {
+                if (cursor_live(ci, sc)) {
+                    if (issuer) {
+                        fence_async_smem();
+                        issue((k - 1) % NS);
+                    }
+                    ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+                }
+                if (warp == 0) store_item_comp(red[(k - 1) & 1], 0, part, 0, prev);
+            }
+            acc = compute_a2(T, li, P, pvec, stages + s * SB, Pn);
+        } else {
+            acc = compute_b(T, li, P, salpha(sc, st, cc.t), flag, stages + s * SB);
+        }
+        for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+        if (lane == 0) red[k & 1][0][warp] = acc;
+        prev = T.item0 + li;
+        if (KIND == 1) {
+            __syncthreads();
+            if (cursor_live(ci, sc)) {
+                if (issuer) {
+                    fence_async_smem();
+                    issue(s);
+                }
+                ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+            }
+            if (sums && warp == 0) store_item_comp(red[k & 1], 0, part, 0, prev);
+        }
+        ++k;
+        cc = cursor_next(cc, sc, gt, st, ntiles, rev);
+    }
+    __syncthreads();
+    if (KIND == 0 && warp == 0) store_item_comp(red[(k - 1) & 1], 0, part, 0, prev);
+    __syncthreads();
+    if (!sums) return;
+    /* the block's partials of every active tile of its slice are stored */
+    for (int t = sc.t0; t <= sc.t1; ++t) {
+        if (sc.pre[t + 1] == sc.pre[t] || !sactive(sc, st, t)) continue;
+        const TileDesc &T = stile(sc, gt, t);
+        int a, b;
+        slice_items(sc, T, t, a, b);
+        if (b > a) seg_done(T, t, b - a, part, tot, cnt, sw, s_bcast, s_flag);
+    }
+    __syncthreads();
 }
 
 template <int NS>
@@ -1222,7 +1246,7 @@ __global__ void __launch_bounds__(kItemThreads, MINB)
 {
     extern __shared__ __align__(128) char dsm_raw[];
     __shared__ double sw[32];
-    __shared__ double red[2][kNComp][8];   /* mixed: warp partials by item parity */
+    __shared__ double red[2][kNComp][8];   /* warp partials by item parity */
     __shared__ double sgrp[kItemGroup][8];   /* warp sums of a group of items */
     __shared__ double s_bcast;
     __shared__ int s_flag;
@@ -1304,8 +1328,8 @@ __global__ void __launch_bounds__(kItemThreads, MINB)
                 }
                 __syncthreads();
                 run_pass<0, NS>(sc, tiles, stA, ntiles, P, M, it & 1, pnew, it == 0, pbuf[pc & 1],
-                            tbuf[pc & 1], tick, sw, &s_bcast, &s_flag, (double *)Pn, dsm, bars,
-                            parity, ctl, timeout_ns, false);
+                            tbuf[pc & 1], tick, sw, red, &s_bcast, &s_flag, (double *)Pn, dsm,
+                            bars, parity, ctl, timeout_ns, false);
                 ++pc;
                 if (!grid_sync(ctl, timeout_ns)) return;
                 if (*(volatile int *)&ctl->snap <= 0) break;
@@ -1330,8 +1354,8 @@ __global__ void __launch_bounds__(kItemThreads, MINB)
                 }
                 __syncthreads();
                 run_pass<1, NS>(sc, tiles, stB, ntiles, P, M, (it + 1) & 1, pnew, true, pbuf[pc & 1],
-                            tbuf[pc & 1], tick, sw, &s_bcast, &s_flag, (double *)Pn, dsm, bars,
-                            parity, ctl, timeout_ns, true);
+                            tbuf[pc & 1], tick, sw, red, &s_bcast, &s_flag, (double *)Pn, dsm,
+                            bars, parity, ctl, timeout_ns, true);
                 ++pc;
                 if (!grid_sync(ctl, timeout_ns)) return;
                 ++it;
