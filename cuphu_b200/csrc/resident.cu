@@ -31,18 +31,19 @@
  *  - Every wait is bounded: when it runs out the error status is set, which
  *    ends all other waits, and the kernel returns.
  *
- * What bounds it (967 x 967, 144 blocks of 7 x 1 items, 13.6 k cycles =
- * 6.6 us per iteration; k_solve took 25 us): the exchange 4.8 k cycles from
- * the last store to the totals, of which 1.3 k are the least that one store
- * and one load of a line another SM has just written take; the second half
- * 5.4 k, bound by instruction issue (about 330 warp instructions per item,
- * 80 of them register moves and addresses, and 20 FP32-to-FP64 conversions at
- * a quarter of the issue rate); the first half 1.3 k, sending 1.0 k, the
- * scalars 0.6 k.  Regions instead of items dealt out by the slots of
- * k_solve's reduction tree cut the rims of this tile from 1280 to 352 pixels
- * per block, use all SMs, and took 8.2 us to 6.6; one FP64 sum per thread
- * instead of a warp tree per item and FP32 products split by FMA are part of
- * that.  At 512 x 512 (2 items per block) 4.4 us, at 96 x 128 (1 item) 2.7.
+ * What bounds it (967 x 967, 144 blocks of 7 x 1 items, 11.0 k cycles =
+ * 5.5 us per iteration; k_solve took 25 us): the second half 5.0 k, bound by
+ * instruction issue (about 300 warp instructions per item, 80 of them register
+ * moves and addresses, and 20 FP32-to-FP64 conversions at a quarter of the
+ * issue rate); the exchange 2.5 k from the last store to the totals, of which
+ * 1.3 k are the least that one store and one load of a line another SM has
+ * just written take; the first half 1.3 k, sending 1.2 k, the scalars 0.6 k.
+ * Regions instead of items dealt out by the slots of k_solve's reduction tree
+ * cut the rims of this tile from 1280 to 352 pixels per block and use all
+ * SMs, and one FP64 sum per thread replaces a warp tree per item over FP32
+ * products split by FMA: 8.2 -> 6.6 us, the rest is the exchange's polling
+ * (poll_together).  512 x 512 (2 items per block): 3.3 us, k_solve 15.8;
+ * 96 x 128 (1 item): 2.7, k_solve 12.7.
  */
 #include "resident.cuh"
 
@@ -208,11 +209,11 @@ __device__ __forceinline__ ulonglong2 *mail_of(int block, unsigned seq, int m, i
 
 /* Sum the threads' values over the block and send the sums to every block of
  * the group.  A block stores its packets into every mailbox, its own
- * included (8 KB per block and exchange for 128 blocks): one hop.  Measured
- * for 128 blocks, from the stores to the totals: 1900 cycles, against 4900
- * when one block per component collects and publishes (two hops) and 7500
- * when every block polls the members' own copies (128 readers of each
- * line). */
+ * included (8 KB per block and exchange for 128 blocks): one hop.  An
+ * iteration at 512 x 512 (128 blocks) takes 3.3 us; with two hops over a grid
+ * of 12 x 11 blocks (one warp, few messages) 4.1, and more with a block per
+ * component that collects and publishes, or with every block polling the
+ * members' own copies (128 readers of each line). */
 template <int NCOMP>
 __device__ __forceinline__ void send_sums(const ResCtx &C, const double acc[kNComp], unsigned seq)
 {
@@ -239,19 +240,6 @@ __device__ __forceinline__ void send_sums(const ResCtx &C, const double acc[kNCo
                          (unsigned long long)__double_as_longlong(v), (unsigned long long)seq);
 }
 
-/* wait for a packet of exchange `seq` that was asked for into (lo, hi) */
-__device__ __forceinline__ bool packet_wait(const ulonglong2 *p, unsigned seq,
-                                            unsigned long long &lo, unsigned long long hi)
-{
-    if (hi == (unsigned long long)seq) return true;
-    Waiter w(res_shared().K.ctl, res_shared().K.sp.timeout_ns);
-    do {
-        if (!w.turn()) return false;
-        packet_load(p, lo, hi);
-    } while (hi != (unsigned long long)seq);
-    return true;
-}
-
 /* The sums of exchange `seq` over the group, in warp 0 (every block adds the
  * members' partials in the same order).  Thread t polls packets t and t + 512
  * of its block's mailbox. */
@@ -259,20 +247,23 @@ template <int NCOMP>
 __device__ __forceinline__ bool totals(const ResCtx &C, unsigned seq, double out[NCOMP])
 {
     ResShared &sh = res_shared();
-    const int c = C.lane & 3;
+    const int c = C.lane & 3, cc = c < NCOMP ? c : 0, n = (int)sh.nact;
+    const int m = threadIdx.x >> 2, m2 = m + kResThreads / 4;
     bool ok = true;
     double v = 0.0;
-    if (c < NCOMP) {
-        const int m = threadIdx.x >> 2, m2 = m + kResThreads / 4, n = (int)sh.nact;
-        const ulonglong2 *p = mail_of(blockIdx.x, seq, m, c);
-        const ulonglong2 *p2 = p + kResThreads;
-        unsigned long long lo = 0, hi = seq, lo2 = 0, hi2 = seq;
-        if (m < n) packet_load(p, lo, hi);
-        if (m2 < n) packet_load(p2, lo2, hi2);
-        ok = packet_wait(p, seq, lo, hi) && packet_wait(p2, seq, lo2, hi2);
-        v = __longlong_as_double((long long)lo) + __longlong_as_double((long long)lo2);
+    if (8 * C.warp < n) {
+        const bool n0 = m < n, n1 = m2 < n, two = 8 * C.warp + kResThreads / 4 < n;
+        const ulonglong2 *p0 = mail_of(blockIdx.x, seq, n0 ? m : 0, cc);
+        const ulonglong2 *p1 = mail_of(blockIdx.x, seq, n1 ? m2 : 0, cc);
+        unsigned long long a0, b0, a1 = 0, b1 = seq;
+        ok = poll_together(sh, [&] {
+            packet_load(p0, a0, b0);
+            if (two) packet_load(p1, a1, b1);
+            return (!n0 || b0 == (unsigned long long)seq) && (!n1 || b1 == (unsigned long long)seq);
+        });
+        if (n0 && c < NCOMP) v = __longlong_as_double((long long)a0);
+        if (n1 && c < NCOMP) v += __longlong_as_double((long long)a1);
     }
-    __syncwarp();
 #pragma unroll
     for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     if (C.lane < NCOMP) sh.own.tot[C.warp][C.lane] = v;

@@ -24,10 +24,10 @@
  * the first 8 - g levels of that butterfly stay inside a block: a block
  * publishes one partial, and every block finishes the tree for itself.
  *
- * What bounds it: two exchanges of about 2.5 us each per iteration (see
- * resident.cu), and with 8 items per block the shared-memory and tensor-memory
- * latency of the two halves.  Per iteration 6.8 us at 256 x 256, 8.7 us at
- * 512 x 512, 14.2 us at 967 x 967; the streaming form took 22, 28 and 50 us.
+ * What bounds it: two exchanges per iteration (see resident.cu), and with 8
+ * items per block the shared-memory and tensor-memory latency of the two
+ * halves.  Per iteration 5.5 us at 256 x 256, 6.2 us at 512 x 512, 11.1 us at
+ * 967 x 967; the streaming form took 22, 28 and 50 us.
  */
 #include "resident_geom.cuh"
 
@@ -36,7 +36,6 @@ namespace {
 constexpr int kResItems = kResItems64;
 struct ResOwn {
     double red[kResItems][8];           /* warp sums per item */
-    double part;                        /* the block's partial */
     double tot[16];                     /* warp sums of an exchange */
     unsigned nbr[kResItems][4];         /* packet base of the rim sources: above,
                                            below, left, right (~0: outside) */
@@ -201,22 +200,24 @@ __device__ __forceinline__ double quotient_pos(double a, double b)
     return (q * back) * sb;
 }
 
-/* A block's mailbox: [parity][member m] packets, 64 bytes apart: two writers
- * in one 32-byte sector cost an iteration at 512^2 1.3 us */
-constexpr int kMailStep = 4;
-constexpr int kMailN = 2 * kResMembers * kMailStep;
+/* A block's mailbox: [parity][member m] packets, four copies of each (64
+ * bytes): four lanes store and read one packet, whole sectors at a time.
+ * (With one lane in four: 7.9 us per iteration at 512 x 512 instead of 6.2.) */
+constexpr int kCopies = 4;
+constexpr int kMailN = 2 * kResMembers * kCopies;
 __device__ __forceinline__ ulonglong2 *mail_of(int block, unsigned seq, int m)
 {
-    return res_shared().K.A.mail + (size_t)block * kMailN + ((seq & 1u) * kResMembers + m) * kMailStep;
+    return res_shared().K.A.mail + (size_t)block * kMailN +
+           ((seq & 1u) * kResMembers + m) * kCopies + (threadIdx.x & 3);
 }
 
-/* The block's partial into own.part: warp 0 forms the items' partials (lanes
- * 2 i + h hold the half tree of warp parity h), then the slot sums (items of
- * a slot in order) and the butterfly levels inside the block. */
-__device__ __forceinline__ void block_partial(const ResCtx &C)
+/* The block's partial, after a barrier that follows the items' warp sums: the
+ * items' partials (lanes 2 i + h hold the half tree of warp parity h), the
+ * slot sums (items of a slot in order) and the butterfly levels inside the
+ * block.  Every warp forms it, so that all can send it at once. */
+__device__ __forceinline__ double block_partial(const ResCtx &C)
 {
-    if (C.warp != 0) return;
-    ResOwn &own = res_shared().own;
+    const ResOwn &own = res_shared().own;
     const int i = C.lane >> 1, h = C.lane & 1, nloc = res_shared().nloc;
     double v = 0.0;
     if (i < nloc) {
@@ -231,49 +232,42 @@ __device__ __forceinline__ void block_partial(const ResCtx &C)
         if (k + sub < nloc) a += x;
     }
     for (int off = S >> 1; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-    if (C.lane == 0) own.part = a;
+    return a;
 }
 
-/* Send the block's partial to every block of the group: thread 4 d to member
- * d's mailbox (spread over all warps: a warp's store goes to eight blocks). */
-__device__ __forceinline__ void send_partial(unsigned seq)
+/* Send the block's partial to every block of the group: threads 4 d .. 4 d + 3
+ * to member d's mailbox. */
+__device__ __forceinline__ void send_partial(double v, unsigned seq)
 {
-    __syncthreads();
     const ResShared &sh = res_shared();
     const int d = threadIdx.x >> 2;
-    if ((threadIdx.x & 3) == 0 && d < (1 << sh.own.g) && sh.phys[d] != 0xffffu)
+    if (d < (1 << sh.own.g) && sh.phys[d] != 0xffffu)
         packet_store(mail_of(sh.phys[d], seq, sh.member),
-                     (unsigned long long)__double_as_longlong(sh.own.part),
-                     (unsigned long long)seq);
+                     (unsigned long long)__double_as_longlong(v), (unsigned long long)seq);
 }
 
 /* Wait for exchange `seq` and finish the tree; the total is returned in warp
- * 0.  One hop: every member stores its packet into every mailbox, and thread
- * 32 w + 4 h polls the packet of member 16 h + w of its own block's mailbox.
- * The members' bits combine from the top: three levels across the lanes,
- * four across the warps. */
+ * 0.  One hop: every member stores its packet into every mailbox, and threads
+ * 32 w + 4 h .. + 3 poll the packet of member 16 h + w of their block's
+ * mailbox.  The members' bits combine from the top: three levels across the
+ * lanes, four across the warps. */
 __device__ __forceinline__ bool total(const ResCtx &C, unsigned seq, double &out)
 {
     ResShared &sh = res_shared();
     bool ok = true;
     const int m = ((C.lane >> 2) << 4) | C.warp;
-    unsigned long long lo = 0;
-    if ((C.lane & 3) == 0 && m < (1 << sh.own.g) && sh.phys[m] != 0xffffu) {
-        const ulonglong2 *p = mail_of(blockIdx.x, seq, m);
-        unsigned long long hi;
-        packet_load(p, lo, hi);
-        if (hi != (unsigned long long)seq) {
-            Waiter w(sh.K.ctl, sh.K.sp.timeout_ns);
-            do {
-                if (!w.turn()) {
-                    ok = false;
-                    break;
-                }
-                packet_load(p, lo, hi);
-            } while (hi != (unsigned long long)seq);
-        }
+    unsigned long long lo = 0, hi;
+    const bool need = m < (1 << sh.own.g) && sh.phys[m] != 0xffffu;
+    const unsigned who = __ballot_sync(0xffffffffu, need);
+    if (who) {
+        const int any = __shfl_sync(0xffffffffu, m, __ffs(who) - 1);
+        const ulonglong2 *p = mail_of(blockIdx.x, seq, need ? m : any);
+        ok = poll_together(sh, [&] {
+            packet_load(p, lo, hi);
+            return hi == (unsigned long long)seq;
+        });
+        if (!need) lo = 0;
     }
-    __syncwarp();
     double v = __longlong_as_double((long long)lo);
 #pragma unroll
     for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -628,8 +622,7 @@ __device__ __noinline__ bool iterate()
             item_sum(C, i, acc);
         }
         __syncthreads();
-        block_partial(C);
-        send_partial(++seq);
+        send_partial(block_partial(C), ++seq);
         double tot;
         if (!total(C, seq, tot)) return false;
         if (threadIdx.x == 0) {
@@ -682,8 +675,7 @@ __device__ __noinline__ bool iterate()
         odd = __syncthreads_or(odd);
         if (odd) slow_update(seq);
         if (threadIdx.x == 0) sh.own.slow = odd;
-        block_partial(C);
-        send_partial(seq);
+        send_partial(block_partial(C), seq);
         rim_ask(C, seq, A);
         if (!total(C, seq, tot)) return false;
         if (threadIdx.x == 0) {
@@ -718,8 +710,7 @@ template <bool WLS> __device__ __noinline__ bool assemble(bool zero_x, double &r
     }
     __syncthreads();
     const unsigned seq = sh.seq + 1;
-    block_partial(C);
-    send_partial(seq);
+    send_partial(block_partial(C), seq);
     if (!total(C, seq, rz)) return false;
     if (threadIdx.x == 0) sh.seq = seq;
     return group_sync();

@@ -73,7 +73,7 @@ Shape region_shape(const TileDesc &T, int k, int nblk)
 void plan_resident(const std::vector<TileDesc> &tiles, int nblk, bool fp64, ResidentPlan &R)
 {
     const int cap = fp64 ? kResItems64 : kResItemsMixed;
-    const double c0 = fp64 ? 7.0 : 3.3, c1 = fp64 ? 0.9 : 0.42;
+    const double c0 = fp64 ? 4.8 : 2.4, c1 = fp64 ? 0.78 : 0.42;
     R = ResidentPlan();
     /* the split of tile t under the bound k, or the nearest one above it */
     auto shape = [&](int t, int k) {
