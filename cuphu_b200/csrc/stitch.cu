@@ -11,13 +11,16 @@
  * running maximum label of the preceding tiles.  The Python reference-pixel
  * shift (_unwrap.py:605-617) is applied in the same merge pass.
  *
- * B200 design: one CTA per tile pair finds the weighted median by a 4-pass
- * radix select over the order-preserving 32-bit key of the float
- * differences, with weights accumulated as exact 2^-28 fixed point (every
- * coherence weight >= 0.05 is an exact multiple of 2^-28, so the sums equal
- * the reference's double accumulation exactly); no sort, no host copy.
+ * B200 design: a cluster of eight CTAs per tile pair finds the weighted median
+ * by a 3-pass radix select (11, 11 and 10 bits) over the order-preserving
+ * 32-bit key of the float differences, with weights accumulated as exact 2^-28
+ * fixed point (every coherence weight >= 0.05 is an exact multiple of 2^-28, so
+ * the sums equal the reference's double accumulation exactly); no sort, no host
+ * copy, no workspace: the histograms are added up over the cluster's shared memory.
  */
 #include "kernels.cuh"
+
+#include <cooperative_groups.h>
 
 namespace cuphu {
 
@@ -33,92 +36,191 @@ __device__ __forceinline__ float fkey_inv(uint32_t k)
     return __uint_as_float(u);
 }
 
-struct PairSample {
-    bool ok;
-    uint32_t key;
-    unsigned long long w;
+constexpr int kMedCtas = 8;       /* CTAs per pair, one portable cluster */
+constexpr int kMedThreads = 512;
+constexpr int kMedBins = 2048;
+constexpr int kMedVec = 4;        /* samples per thread and step, 32 columns apart */
+constexpr int kMedSlice = kMedBins / kMedCtas;
+
+/* the pair's overlap: sample (i, j) is A's pixel (ar0 + i, ac0 + j) and B's (i, j) */
+struct PairOverlap {
+    const float *ca, *cb, *ua, *ub;
+    const unsigned char *fa, *fb;   /* confidence masks, or null */
+    size_t pa, pb, qa, qb;          /* row pitches: inputs, unwrapped planes */
+    int n1, n2;
 };
 
-__device__ __forceinline__ PairSample pair_sample(const PairDesc &pd, const TileDesc &A,
-                                                  const TileDesc &B, const SolverPlanes &P,
-                                                  int i, int j)
+/* hist[bin] += w modulo 2^64 from two native 32-bit shared atomics: the carry is read off the
+ * value that the first one returns (a 64-bit shared atomic is a compare-and-swap loop, which the
+ * narrow distribution of the differences makes long) */
+__device__ __forceinline__ void hist_add(uint32_t *lo, uint32_t *hi, uint32_t bin,
+                                         unsigned long long w)
 {
-    PairSample s;
-    s.ok = false;
-    int ar, ac, br, bc;
-    if (pd.dir == 0) { ar = i; ac = A.nc - pd.ov + j; br = i; bc = j; }
-    else             { ar = A.nr - pd.ov + i; ac = j; br = i; bc = j; }
-    size_t ga = (size_t)ar * A.ph_pitch + ac, gb = (size_t)br * B.ph_pitch + bc;
-    float ca = sane(A.corr[ga]), cb = sane(B.corr[gb]);
-    if (ca < 0.05f || cb < 0.05f) return s;
-    if (A.conf && !A.conf[ga]) return s;
-    if (B.conf && !B.conf[gb]) return s;
-    float ua = P.unw[A.pix + (size_t)ar * A.pitch + ac];
-    float ub = P.unw[B.pix + (size_t)br * B.pitch + bc];
-    s.ok = true;
-    s.key = fkey(ua - ub);
-    float w = ca < cb ? ca : cb;
-    s.w = (unsigned long long)((double)w * 268435456.0);
-    return s;
+    const uint32_t wl = (uint32_t)w, old = atomicAdd(lo + bin, wl);
+    const uint32_t wh = (uint32_t)(w >> 32) + (old + wl < old ? 1u : 0u);
+    if (wh) atomicAdd(hi + bin, wh);
 }
 
-__global__ void __launch_bounds__(256) k_pair_median(const PairDesc *__restrict__ pairs,
-                                                     const TileDesc *__restrict__ tiles,
-                                                     SolverPlanes P, double *pair_k)
+/* one sample of every lane (all 32 are here).  The lanes that share the first counting lane's bin
+ * are added up in registers first: in the upper digits that is nearly the whole warp. */
+__device__ __forceinline__ void warp_hist(uint32_t *lo, uint32_t *hi, bool ok, uint32_t bin,
+                                          unsigned long long w)
 {
-    __shared__ unsigned long long hist[256];
-    __shared__ unsigned long long s_total, s_below;
-    __shared__ uint32_t s_prefix, s_mask;
-    const PairDesc pd = pairs[blockIdx.x];
+    const unsigned live = __ballot_sync(0xffffffffu, ok);
+    if (live == 0u) return;
+    const int first = __ffs(live) - 1;
+    const uint32_t lead = __shfl_sync(0xffffffffu, bin, first);
+    const bool same = ok && bin == lead;
+    const unsigned long long ws = same ? w : 0ull;
+    /* 24 + 24 + 16 bits: 32 lanes cannot overflow 32 bits, and the total is exact modulo 2^64 */
+    const uint32_t s0 = __reduce_add_sync(0xffffffffu, (uint32_t)(ws & 0xFFFFFFull));
+    const uint32_t s1 = __reduce_add_sync(0xffffffffu, (uint32_t)(ws >> 24) & 0xFFFFFFu);
+    const uint32_t s2 = __reduce_add_sync(0xffffffffu, (uint32_t)(ws >> 48));
+    if ((int)(threadIdx.x & 31u) == first)
+        hist_add(lo, hi, bin, (unsigned long long)s0 + ((unsigned long long)s1 << 24) +
+                                  ((unsigned long long)s2 << 48));
+    else if (ok && !same)
+        hist_add(lo, hi, bin, w);
+}
+
+/* the differences whose key agrees with `prefix` under `mask`, into the CTA's histogram */
+__device__ __forceinline__ void pair_pass(const PairOverlap &o, uint32_t *lo, uint32_t *hi,
+                                          uint32_t prefix, uint32_t mask, int shift, uint32_t digit,
+                                          unsigned rank)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned nwarps = kMedCtas * kMedThreads / 32;
+    const unsigned nb = ((unsigned)o.n2 + 32u * kMedVec - 1u) / (32u * kMedVec);
+    const unsigned units = nb * (unsigned)o.n1;
+    for (unsigned u = rank * (kMedThreads / 32) + (threadIdx.x >> 5); u < units; u += nwarps) {
+        const int i = (int)(u / nb), j0 = (int)(u % nb) * 32 * kMedVec + lane;
+        float ca[kMedVec], cb[kMedVec], ua[kMedVec], ub[kMedVec];
+        bool ok[kMedVec];
+#pragma unroll
+        for (int v = 0; v < kMedVec; ++v) {
+            const int j = j0 + 32 * v;
+            ca[v] = cb[v] = ua[v] = ub[v] = 0.0f;
+            ok[v] = j < o.n2;
+            if (!ok[v]) continue;
+            ca[v] = o.ca[(size_t)i * o.pa + j];
+            cb[v] = o.cb[(size_t)i * o.pb + j];
+            ua[v] = o.ua[(size_t)i * o.qa + j];
+            ub[v] = o.ub[(size_t)i * o.qb + j];
+            if (o.fa) ok[v] = o.fa[(size_t)i * o.pa + j] != 0;
+            if (o.fb) ok[v] = ok[v] && o.fb[(size_t)i * o.pb + j] != 0;
+        }
+#pragma unroll
+        for (int v = 0; v < kMedVec; ++v) {
+            const float a = sane(ca[v]), b = sane(cb[v]);
+            const uint32_t key = fkey(ua[v] - ub[v]);
+            const bool in = ok[v] && !(a < 0.05f || b < 0.05f) && (key & mask) == prefix;
+            const float w = a < b ? a : b;
+            /* a power of two: the product is exact, as in 64 bits */
+            warp_hist(lo, hi, in, (key >> shift) & digit,
+                      in ? (unsigned long long)(w * 268435456.0f) : 0ull);
+        }
+    }
+}
+
+/* Latency-bound at one CTA per pair: 16.25 ms for the one pair of a 2051 x 1537 scene, five passes
+ * of 256 threads with one load chain each and a 64-bit compare-and-swap histogram that the narrow
+ * distribution serialised.  Sixteen times the threads, four samples in flight each, three passes
+ * (the total is the first histogram's sum) and register sums for the crowded bin: 0.050 ms. */
+__global__ void __cluster_dims__(kMedCtas, 1, 1) __launch_bounds__(kMedThreads)
+    k_pair_median(const PairDesc *__restrict__ pairs, const TileDesc *__restrict__ tiles,
+                  SolverPlanes P, double *pair_k)
+{
+    namespace cg = cooperative_groups;
+    __shared__ uint32_t s_lo[kMedBins], s_hi[kMedBins];
+    __shared__ unsigned long long s_tot[kMedBins];     /* the pair's histogram, in every CTA */
+    __shared__ unsigned long long s_warp[kMedThreads / 32];
+    __shared__ unsigned long long s_below;
+    __shared__ int s_sel;
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank();
+    const unsigned pair = blockIdx.x / kMedCtas;
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const PairDesc pd = pairs[pair];
     const TileDesc &A = tiles[pd.a];
     const TileDesc &B = tiles[pd.b];
     bool valid = pd.ov > 0 && (pd.dir == 0 ? (pd.ov <= A.nc && pd.ov <= B.nc)
                                           : (pd.ov <= A.nr && pd.ov <= B.nr));
-    if (!valid) {
-        if (threadIdx.x == 0) pair_k[blockIdx.x] = 0.0;
+    if (!valid) {   /* the same in all CTAs of the cluster */
+        if (rank == 0 && t == 0) pair_k[pair] = 0.0;
         return;
     }
-    int n1 = pd.dir == 0 ? min(A.nr, B.nr) : pd.ov;
-    int n2 = pd.dir == 0 ? pd.ov : min(A.nc, B.nc);
-    long long ns = (long long)n1 * n2;
-    if (threadIdx.x == 0) { s_total = 0ull; s_below = 0ull; s_prefix = 0u; s_mask = 0u; }
-    __syncthreads();
-    unsigned long long loc = 0ull;
-    for (long long k = threadIdx.x; k < ns; k += blockDim.x) {
-        PairSample s = pair_sample(pd, A, B, P, (int)(k / n2), (int)(k % n2));
-        if (s.ok) loc += s.w;
-    }
-    atomicAdd(&s_total, loc);
-    __syncthreads();
-    unsigned long long total = s_total;
-    if (total == 0ull) {
-        if (threadIdx.x == 0) pair_k[blockIdx.x] = 0.0;
-        return;
-    }
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        hist[threadIdx.x] = 0ull;
+    PairOverlap o;
+    o.n1 = pd.dir == 0 ? min(A.nr, B.nr) : pd.ov;
+    o.n2 = pd.dir == 0 ? pd.ov : min(A.nc, B.nc);
+    const size_t ar0 = pd.dir == 0 ? 0 : A.nr - pd.ov, ac0 = pd.dir == 0 ? A.nc - pd.ov : 0;
+    o.pa = A.ph_pitch; o.pb = B.ph_pitch; o.qa = A.pitch; o.qb = B.pitch;
+    o.ca = A.corr + ar0 * o.pa + ac0; o.cb = B.corr;
+    o.fa = A.conf ? A.conf + ar0 * o.pa + ac0 : nullptr; o.fb = B.conf;
+    o.ua = P.unw + A.pix + ar0 * o.qa + ac0; o.ub = P.unw + B.pix;
+
+    unsigned long long total = 0ull, below = 0ull;
+    uint32_t prefix = 0u, mask = 0u;
+    for (int pass = 0; pass < 3; ++pass) {
+        const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+        const uint32_t digit = pass == 2 ? 1023u : 2047u;
+        for (int b = t; b < kMedBins; b += kMedThreads) { s_lo[b] = 0u; s_hi[b] = 0u; }
         __syncthreads();
-        uint32_t prefix = s_prefix, mask = s_mask;
-        for (long long k = threadIdx.x; k < ns; k += blockDim.x) {
-            PairSample s = pair_sample(pd, A, B, P, (int)(k / n2), (int)(k % n2));
-            if (s.ok && (s.key & mask) == prefix)
-                atomicAdd(&hist[(s.key >> shift) & 255u], s.w);
+        pair_pass(o, s_lo, s_hi, prefix, mask, shift, digit, rank);
+        cluster.sync();
+        /* each CTA adds up its slice of the bins over the cluster and hands it to all */
+        if (t < kMedSlice) {
+            const int b = (int)rank * kMedSlice + t;
+            unsigned long long sum = 0ull;
+            for (int c = 0; c < kMedCtas; ++c)
+                sum += cluster.map_shared_rank(s_lo, c)[b] +
+                       ((unsigned long long)cluster.map_shared_rank(s_hi, c)[b] << 32);
+            for (int c = 0; c < kMedCtas; ++c) cluster.map_shared_rank(s_tot, c)[b] = sum;
         }
+        cluster.sync();   /* also the last access to another CTA's histogram in this pass */
+
+        /* exclusive prefix of the thread's bins over the CTA */
+        constexpr int kPer = kMedBins / kMedThreads;
+        unsigned long long mine = 0ull;
+        for (int k = 0; k < kPer; ++k) mine += s_tot[t * kPer + k];
+        unsigned long long incl = mine;
+        for (int off = 1; off < 32; off <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += y;
+        }
+        if (lane == 31) s_warp[wp] = incl;
+        if (t == 0) s_sel = (int)digit;   /* stays only if the weights overflow 63 bits */
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long below = s_below;
-            int sel = 255;
-            for (int b = 0; b < 256; ++b) {
-                if (2ull * (below + hist[b]) >= total) { sel = b; break; }
-                below += hist[b];
+        unsigned long long before = below, all = 0ull;
+        for (int k = 0; k < kMedThreads / 32; ++k) {
+            if (k < wp) before += s_warp[k];
+            all += s_warp[k];
+        }
+        before += incl - mine;
+        if (pass == 0) {
+            total = all;
+            if (total == 0ull) {   /* the same in all CTAs */
+                if (rank == 0 && t == 0) pair_k[pair] = 0.0;
+                return;
             }
-            s_below = below;
-            s_prefix = prefix | ((uint32_t)sel << shift);
-            s_mask = mask | (255u << shift);
         }
+        /* the first bin at which twice the weight up to it reaches the total */
+        unsigned long long run = before;
+        int sel = -1;
+        for (int k = 0; k < kPer; ++k) {
+            const unsigned long long next = run + s_tot[t * kPer + k];
+            if (2ull * next >= total) { sel = t * kPer + k; break; }
+            run = next;
+        }
+        if (sel >= 0) atomicMin(&s_sel, sel);
+        if (t == 0) s_below = below + all;
         __syncthreads();
+        if (sel >= 0 && s_sel == sel) s_below = run;
+        __syncthreads();
+        below = s_below;
+        prefix |= (uint32_t)s_sel << shift;
+        mask |= digit << shift;
     }
-    if (threadIdx.x == 0) pair_k[blockIdx.x] = (double)fkey_inv(s_prefix) / kTwoPiD;
+    if (rank == 0 && t == 0) pair_k[pair] = (double)fkey_inv(prefix) / kTwoPiD;
 }
 
 /* one thread per scene: BFS tile offsets, label offsets, reference shift */
@@ -252,7 +354,8 @@ int launch_stitch(const ScenePlan *scenes, int nscenes, const TileDesc *tiles,
                   const int *ntile_labels, double *pair_k, double *tile_k,
                   unsigned *comp_off, SceneOut *sout, cudaStream_t s)
 {
-    if (npairs > 0) k_pair_median<<<npairs, 256, 0, s>>>(pairs, tiles, P, pair_k);
+    if (npairs > 0)
+        k_pair_median<<<npairs * kMedCtas, kMedThreads, 0, s>>>(pairs, tiles, P, pair_k);
     /* the BFS queue reuses pair_k's tail: [npairs] medians, then [ntiles] queue */
     int *queue = reinterpret_cast<int *>(pair_k + npairs);
     k_stitch_finalize<<<(nscenes + 63) / 64, 64, 0, s>>>(scenes, nscenes, tiles, P, ntile_labels,

@@ -350,3 +350,36 @@ def test_regrow_conncomp_gpu():
 def test_gpu_info():
     info = cuphu.gpu_info(0)
     assert info["total_memory"] > 0 and "B200" in info["name"] or info["total_memory"] > 0
+
+
+@pytest.mark.parametrize("ntiles,ovl,conf", [((1, 2), (0, 1), False), ((1, 2), (0, 127), False),
+                                             ((1, 2), (0, 129), True), ((2, 1), (96, 0), True),
+                                             ((3, 3), (33, 40), False), ((1, 2), (0, 60), None)])
+def test_registration_medians_over_narrow_and_wide_overlaps(torch_cuda, ntiles, ovl, conf):
+    """Each pair's weighted median, at overlaps on both sides of a warp's 128 samples, with a
+    confidence mask, and (conf None) with no coherent sample in the overlap; bit for bit."""
+    nr, nc = (310, 150) if ntiles[0] > 1 else (70, 390)
+    if ntiles == (3, 3):
+        nr, nc = 190, 230
+    ig, g, _, _ = S.bumps(nr, nc, seed=17, nbumps=4, amp_range=(20, 40), sigma_range=(8, 20))
+    ph = O.phase_from_igram(ig)
+    g = g.copy()
+    cm = None
+    if conf:
+        cm = (np.random.default_rng(5).uniform(size=g.shape) > 0.4).astype(np.uint8)
+    if conf is None:
+        g[:, 150:240] = 0.03
+    want_u, want_c, _ = O.unwrap_tiled(ph, g, 5.0, mode=0, conf_mask=cm, ntiles=ntiles,
+                                       overlap=ovl, opts=O.lap_opts(n_irls=1, max_iter=40))
+    dph, dg = to_dev(ph), to_dev(g)
+    dcf = to_dev(cm) if cm is not None else None
+    du, dc = empty((nr, nc), torch_cuda.float32), empty((nr, nc), torch_cuda.int32)
+    p = default_params(nlooks=5.0, ncorrlooks=5.0)
+    t = default_tile_params(ntilerow=ntiles[0], ntilecol=ntiles[1], rowovrlp=ovl[0],
+                            colovrlp=ovl[1])
+    o = default_solve_options(precision=1, n_irls=1, max_iter=40, ref_row=-1, ref_col=-1)
+    check(lib().cuphu_unwrap_device(None, dptr(dph), dptr(dg), None, dptr(dcf), nr, nc, 0,
+                                    C.byref(p), C.byref(t), C.byref(o), dptr(du), dptr(dc), None,
+                                    None, None))
+    assert np.array_equal(to_host(du).view(np.int32), want_u.view(np.int32))
+    assert np.array_equal(to_host(dc).view(np.uint32), want_c)
