@@ -258,6 +258,33 @@ def test_conncomp_large_random_matches_oracle(torch_cuda):
     assert np.array_equal(to_host(dl).view(np.uint32), want)
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (1, 200), (200, 1), (15, 63), (16, 64), (17, 65), (33, 130)])
+@pytest.mark.parametrize("kind", ["noise", "snake", "comb"])
+def test_conncomp_across_item_borders(torch_cuda, shape, kind):
+    """Shapes on both sides of a 16 x 64 work item; speckle, one component that winds through
+    every item (long chains of links), and teeth that meet only in the last row."""
+    nr, nc = shape
+    rng = np.random.default_rng(13)
+    r, c = np.mgrid[0:nr, 0:nc]
+    unw = (0.2 * r + 0.1 * c).astype(np.float32)
+    corr = np.ones(shape, np.float32)
+    if kind == "noise":
+        unw += (2 * np.pi * rng.integers(0, 2, shape)).astype(np.float32)
+        corr = rng.uniform(0.0, 0.4, shape).astype(np.float32)
+    elif kind == "snake":
+        corr[(r % 2 == 1) & (c != np.where(r % 4 == 1, nc - 1, 0))] = 0.0
+    else:
+        corr[(c % 2 == 1) & (r != nr - 1)] = 0.0
+    kw = dict(minfrac=0.0, maxncomps=1 << 20)
+    want = O.conncomp(unw, corr, **kw)
+    p = default_params(minconncompfrac=0.0, maxncomps=1 << 20)
+    du, dc = to_dev(unw), to_dev(corr)
+    dl = empty(shape, torch_cuda.int32)
+    check(lib().cuphu_conncomp_gpu(dptr(du), dptr(dc), None, nr, nc, None, None, C.byref(p), 0,
+                                   dptr(dl)))
+    assert np.array_equal(to_host(dl).view(np.uint32), want)
+
+
 @pytest.mark.parametrize("shape", [(37, 45), (1, 70), (70, 1), (129, 300)])
 def test_integrate_matches_oracle_and_reference(torch_cuda, shape):
     nr, nc = shape
