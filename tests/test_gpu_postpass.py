@@ -45,6 +45,20 @@ def test_fix_cycle_spikes_bit_exact_vs_oracle(torch_cuda, shape, seed, mfrac):
     assert np.array_equal(got.view(np.int32), want.view(np.int32))
 
 
+@pytest.mark.parametrize("nl", [2, 3, 33, 1024, 1025, 1026, 2100])
+def test_cycle_spikes_across_block_edges(torch_cuda, nl):
+    """Lines in rows of shifts (a shift changes the next line's decision), on both sides of the
+    1024 lines that are decided together, along rows and along columns."""
+    rng = np.random.default_rng(nl)
+    line = (2 * np.pi * rng.integers(-1, 2, nl)).astype(np.float32)
+    line[1020:1030] = (2 * np.pi * (np.arange(1020, min(nl, 1030)) % 2)).astype(np.float32)
+    unw = np.ascontiguousarray(line[:, None] + rng.normal(0, 0.1, (nl, 24)).astype(np.float32))
+    for u in (unw, np.ascontiguousarray(unw.T)):
+        got = _cuphu_ext._fix_cycle_spikes_test(u)
+        want = O.fix_cycle_spikes(u)
+        assert np.array_equal(got.view(np.int32), want.view(np.int32))
+
+
 def _seamed(nr, nc, ntiles, ovl, seed, mask_frac=0.0):
     rng = np.random.default_rng(seed)
     unw = rng.normal(0, 0.2, (nr, nc)).astype(np.float32)
