@@ -388,11 +388,18 @@ __device__ __forceinline__ void sld4(const double *p, double v[4])
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
+/* What a pass's item loop needs of the tile it is in, in registers: a reference to the block's copy
+ * or, beyond it, the global one is a generic pointer, whose loads are repeated after every store. */
+struct TileView {
+    int nr, nc, pitch, nbx, item0;
+    long long pix;
+};
+
 /* stencil pass on a staged item (FP64, the oracle's operation order), in two
  * halves around the item's barrier.  a1: p_new = z + beta p_old of the own
  * pixels and the halo ring into Pn.  a2: q = A p_new; returns the thread's
  * partial of p.q. */
-__device__ __forceinline__ void compute_a1(const TileDesc &T, int li, bool first, double beta,
+__device__ __forceinline__ void compute_a1(const TileView &T, int li, bool first, double beta,
                                            const char *stage, double *Pn)
 {
     const int r0b = (li / T.nbx) * kItemBy, c0b = (li % T.nbx) * kItemBx;
@@ -431,7 +438,7 @@ __device__ __forceinline__ void compute_a1(const TileDesc &T, int li, bool first
     }
 }
 
-__device__ __forceinline__ double compute_a2(const TileDesc &T, int li, const SolverPlanes &P,
+__device__ __forceinline__ double compute_a2(const TileView &T, int li, const SolverPlanes &P,
                                              double *pnew_all, const char *stage, const double *Pn)
 {
     const int r0b = (li / T.nbx) * kItemBy, c0b = (li % T.nbx) * kItemBx;
@@ -496,7 +503,7 @@ __device__ __forceinline__ void issue_b(const TileDesc &T, int li, const SolveMa
 }
 
 /* update pass (FP64): x += alpha p; r -= alpha q; z = r / diag; partial r.z */
-__device__ __forceinline__ double compute_b(const TileDesc &T, int li, const SolverPlanes &P, double alpha,
+__device__ __forceinline__ double compute_b(const TileView &T, int li, const SolverPlanes &P, double alpha,
                             bool update_r, const char *stage)
 {
     const int r0b = (li / T.nbx) * kItemBy, c0b = (li % T.nbx) * kItemBx;
@@ -581,7 +588,7 @@ struct ItemS {
     size_t o;
 };
 
-__device__ __forceinline__ ItemS item_s(const TileDesc &T, int li, const char *stage)
+__device__ __forceinline__ ItemS item_s(const TileView &T, int li, const char *stage)
 {
     ItemS I;
     I.r0b = (li / T.nbx) * kItemBy;
@@ -607,7 +614,7 @@ __device__ __forceinline__ ItemS item_s(const TileDesc &T, int li, const char *s
     return I;
 }
 
-__device__ __forceinline__ void compute_s1(const TileDesc &T, const ItemS &I, float *rnew_all,
+__device__ __forceinline__ void compute_s1(const TileView &T, const ItemS &I, float *rnew_all,
                                            float *dx_all, bool first, bool fresh, float alphaf,
                                            float betaf, float *Pn, float zn[4], float rd[4],
                                            float rv[4])
@@ -706,7 +713,7 @@ __device__ __forceinline__ void compute_s1(const TileDesc &T, const ItemS &I, fl
     }
 }
 
-__device__ __forceinline__ void compute_s2(const TileDesc &T, const ItemS &I, float *pnew_all,
+__device__ __forceinline__ void compute_s2(const TileView &T, const ItemS &I, float *pnew_all,
                                            float *qnew_all, const float *Pn, const float zn[4],
                                            const float rd[4], const float rv[4], bool fresh,
                                            double acc[kNComp])
@@ -943,50 +950,65 @@ __device__ __forceinline__ void slice_items(const SliceCtl &sc, const TileDesc &
     b = min(sc.s1, sc.pre[t] + T.nitems) - sc.pre[t];
 }
 
-/* position in the slice: counted position p, tile t */
+/* position in the slice: counted position p, tile t, whose items are counted from base to hi (hi =
+ * INT_MIN: past the slice) */
 struct Cursor {
-    int p, t;
+    int p, t, base, hi;
 };
 
 /* Passes walk their slices alternately forwards and backwards: what a pass
  * touched last, the next one reads first, while it is still in the L2
  * (126 MB).  The partials are stored by item, so the order does not show in
- * the sums.  Mixed, one tile, us per iteration always forwards and now: 1600^2
- * 45 -> 17.5, 2048^2 64 -> 27, 4096^2 207 -> 123; FP64 (bound by its item
- * loop, not by memory) unchanged. */
-__device__ __forceinline__ bool cursor_live(Cursor c, const SliceCtl &sc)
-{
-    return c.p >= sc.s0 && c.p < sc.s1;
-}
-/* the next position, from c on, of a tile that is still active */
-__device__ __forceinline__ Cursor cursor_active(Cursor c, const SliceCtl &sc, const TileDesc *g,
+ * the sums.  Mixed, one tile: 2048^2 56.4 -> 54.2 us per iteration, where the
+ * state is a little larger than the L2; 1700 x 1600 (40.6) and 4096^2 (196)
+ * are unchanged, because the passes are bound by their item loops.
+ *
+ * A cursor carries its tile's range and the item loop its tile's description:
+ * looked up for every item, through pointers that may be shared or global,
+ * they cost the mixed passes 10 to 12 % (1700 x 1600 43.9 -> 39.7 us, 2048^2
+ * 60.0 -> 53.8, 4096^2 222 -> 195) and the FP64 ones 2 %. */
+__device__ __forceinline__ bool cursor_live(const Cursor &c) { return c.p < c.hi; }
+/* position p of tile t or, if that tile has ended or is not active, the next one */
+__device__ __forceinline__ Cursor cursor_active(int p, int t, const SliceCtl &sc,
                                                 const TileState *st, int ntiles, bool rev)
 {
     if (rev) {
-        while (c.p >= sc.s0) {
-            while (c.t > 0 && sc.pre[c.t] > c.p) --c.t;
-            if (sactive(sc, st, c.t)) return c;
-            c.p = sc.pre[c.t] - 1;
+        while (p >= sc.s0) {
+            while (t > 0 && sc.pre[t] > p) --t;
+            if (sactive(sc, st, t)) return Cursor{p, t, sc.pre[t], sc.pre[t + 1]};
+            p = sc.pre[t] - 1;
         }
-        return c;
+    } else {
+        while (p < sc.s1) {
+            while (t + 1 <= ntiles && sc.pre[t + 1] <= p) ++t;
+            if (sactive(sc, st, t)) return Cursor{p, t, sc.pre[t], min(sc.pre[t + 1], sc.s1)};
+            p = sc.pre[t + 1];
+        }
     }
-    while (c.p < sc.s1) {
-        while (c.t + 1 <= ntiles && sc.pre[c.t + 1] <= c.p) ++c.t;
-        if (sactive(sc, st, c.t)) return c;
-        c.p = sc.pre[c.t + 1];
-    }
-    return c;
+    return Cursor{p, t, 0, INT_MIN};
 }
-__device__ __forceinline__ Cursor cursor_first(const SliceCtl &sc, const TileDesc *g,
-                                               const TileState *st, int ntiles, bool rev)
+__device__ __forceinline__ Cursor cursor_first(const SliceCtl &sc, const TileState *st, int ntiles,
+                                               bool rev)
 {
-    return cursor_active(rev ? Cursor{sc.s1 - 1, sc.t1} : Cursor{sc.s0, sc.t0}, sc, g, st, ntiles,
-                         rev);
+    return rev ? cursor_active(sc.s1 - 1, sc.t1, sc, st, ntiles, rev)
+               : cursor_active(sc.s0, sc.t0, sc, st, ntiles, rev);
 }
-__device__ __forceinline__ Cursor cursor_next(Cursor c, const SliceCtl &sc, const TileDesc *g,
-                                              const TileState *st, int ntiles, bool rev)
+/* the next position; inside a tile without a look at the slice's tables */
+__device__ __forceinline__ void cursor_next(Cursor &c, const SliceCtl &sc, const TileState *st,
+                                            int ntiles, bool rev)
 {
-    return cursor_active(Cursor{rev ? c.p - 1 : c.p + 1, c.t}, sc, g, st, ntiles, rev);
+    const int p = rev ? c.p - 1 : c.p + 1;
+    if (rev ? p >= max(c.base, sc.s0) : p < c.hi) c.p = p;
+    else c = cursor_active(p, c.t, sc, st, ntiles, rev);
+}
+/* the tile of a cursor, if it is another than before */
+__device__ __forceinline__ void view_tile(TileView &v, int &vt, const Cursor &c, const SliceCtl &sc,
+                                          const TileDesc *g)
+{
+    if (vt == c.t) return;
+    const TileDesc &T = stile(sc, g, c.t);
+    v = TileView{T.nr, T.nc, T.pitch, T.nbx, T.item0, T.pix};
+    vt = c.t;
 }
 
 /* The mixed pass over this block's slice, staged like run_pass but with one
@@ -1032,14 +1054,16 @@ __device__ void run_pass(const SliceCtl &sc, const TileDesc *gt, const TileState
     constexpr size_t PNE = pn_bytes<double>() / sizeof(double);
     const bool sums = KIND == 0 || flag;
     if (sc.s0 >= sc.s1) return;
-    Cursor ci = cursor_first(sc, gt, st, ntiles, rev);
-    if (!cursor_live(ci, sc)) return;
+    Cursor ci = cursor_first(sc, st, ntiles, rev);
+    if (!cursor_live(ci)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool issuer = threadIdx.x == kItemThreads - 32;
     Cursor cc = ci;
+    TileView T;
+    int vt = -1;
     auto issue = [&](int s) {
         const TileDesc &T = stile(sc, gt, ci.t);
-        const int li = ci.p - sc.pre[ci.t];
+        const int li = ci.p - ci.base;
         if (KIND == 0) issue_a(T, li, M, psel, flag, stages + s * SB, bars + s);
         else issue_b(T, li, M, psel, flag, stages + s * SB, bars + s);
     };
@@ -1047,29 +1071,29 @@ __device__ void run_pass(const SliceCtl &sc, const TileDesc *gt, const TileState
         fence_async_global();
         fence_async_smem();
     }
-    for (int k = 0; k < NS && cursor_live(ci, sc); ++k) {
+    for (int k = 0; k < NS && cursor_live(ci); ++k) {
         if (issuer) issue(k);
-        ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+        cursor_next(ci, sc, st, ntiles, rev);
     }
     int k = 0, prev = -1;   /* item number in the pass; item k-1 (stencil pass) */
-    while (cursor_live(cc, sc)) {
+    while (cursor_live(cc)) {
         const int s = k % NS;
         mbar_wait(bars + s, (parity >> s) & 1u, ctl, timeout_ns);
         parity ^= 1u << s;
-        const TileDesc &T = stile(sc, gt, cc.t);
-        const int li = cc.p - sc.pre[cc.t];
+        view_tile(T, vt, cc, sc, gt);
+        const int li = cc.p - cc.base;
         double acc;
         if (KIND == 0) {
             double *Pn = Pn2 + (k & 1) * PNE;
             compute_a1(T, li, flag, sbeta(sc, st, cc.t), stages + s * SB, Pn);
             __syncthreads();
             if (prev >= 0) {
-                if (cursor_live(ci, sc)) {
+                if (cursor_live(ci)) {
                     if (issuer) {
                         fence_async_smem();
                         issue((k - 1) % NS);
                     }
-                    ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+                    cursor_next(ci, sc, st, ntiles, rev);
                 }
                 if (warp == 0) store_item_comp(red[(k - 1) & 1], 0, part, 0, prev);
             }
@@ -1082,17 +1106,17 @@ __device__ void run_pass(const SliceCtl &sc, const TileDesc *gt, const TileState
         prev = T.item0 + li;
         if (KIND == 1) {
             __syncthreads();
-            if (cursor_live(ci, sc)) {
+            if (cursor_live(ci)) {
                 if (issuer) {
                     fence_async_smem();
                     issue(s);
                 }
-                ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+                cursor_next(ci, sc, st, ntiles, rev);
             }
             if (sums && warp == 0) store_item_comp(red[k & 1], 0, part, 0, prev);
         }
         ++k;
-        cc = cursor_next(cc, sc, gt, st, ntiles, rev);
+        cursor_next(cc, sc, st, ntiles, rev);
     }
     __syncthreads();
     if (KIND == 0 && warp == 0) store_item_comp(red[(k - 1) & 1], 0, part, 0, prev);
@@ -1121,29 +1145,31 @@ __device__ void run_pass_s(const SliceCtl &sc, const TileDesc *gt, const TileSta
     constexpr size_t SB = stage_bytes<float>();
     constexpr size_t PNE = pn_bytes<float>() / sizeof(float);
     if (sc.s0 >= sc.s1) return;
-    Cursor ci = cursor_first(sc, gt, st, ntiles, rev);
-    if (!cursor_live(ci, sc)) return;
+    Cursor ci = cursor_first(sc, st, ntiles, rev);
+    if (!cursor_live(ci)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     /* the issuing thread: warp 7, whose post-barrier work is lightest */
     const bool issuer = threadIdx.x == kItemThreads - 32;
     Cursor cc = ci;
+    TileView T;
+    int vt = -1;
     if (issuer) {
         fence_async_global();
         fence_async_smem();
     }
-    for (int k = 0; k < NS && cursor_live(ci, sc); ++k) {
+    for (int k = 0; k < NS && cursor_live(ci); ++k) {
         if (issuer)
-            issue_s(stile(sc, gt, ci.t), ci.p - sc.pre[ci.t], M, zsel, ksel, first, fresh,
+            issue_s(stile(sc, gt, ci.t), ci.p - ci.base, M, zsel, ksel, first, fresh,
                     stages + k * SB, bars + k);
-        ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+        cursor_next(ci, sc, st, ntiles, rev);
     }
     int k = 0, prev = -1;   /* item number in the pass; partial index of item k-1 */
-    while (cursor_live(cc, sc)) {
+    while (cursor_live(cc)) {
         const int s = k % NS;
         mbar_wait(bars + s, (parity >> s) & 1u, ctl, timeout_ns);
         parity ^= 1u << s;
-        const TileDesc &T = stile(sc, gt, cc.t);
-        const int li = cc.p - sc.pre[cc.t];
+        view_tile(T, vt, cc, sc, gt);
+        const int li = cc.p - cc.base;
         const ItemS I = item_s(T, li, stages + s * SB);
         float *Pn = Pn2 + (k & 1) * PNE;
         double acc[kNComp] = {0.0, 0.0, 0.0, 0.0};
@@ -1153,14 +1179,14 @@ __device__ void run_pass_s(const SliceCtl &sc, const TileDesc *gt, const TileSta
                    (float)sbeta(sc, st, cc.t), Pn, zn, rd, rv);
         __syncthreads();
         if (prev >= 0) {
-            if (cursor_live(ci, sc)) {
+            if (cursor_live(ci)) {
                 if (issuer) {
                     const int sp = (k - 1) % NS;
                     fence_async_smem();
-                    issue_s(stile(sc, gt, ci.t), ci.p - sc.pre[ci.t], M, zsel, ksel, first,
+                    issue_s(stile(sc, gt, ci.t), ci.p - ci.base, M, zsel, ksel, first,
                             fresh, stages + sp * SB, bars + sp);
                 }
-                ci = cursor_next(ci, sc, gt, st, ntiles, rev);
+                cursor_next(ci, sc, st, ntiles, rev);
             }
             if (warp < kNComp) store_item_comp(red[(k - 1) & 1], warp, part, nitems, prev);
         }
@@ -1171,7 +1197,7 @@ __device__ void run_pass_s(const SliceCtl &sc, const TileDesc *gt, const TileSta
         }
         prev = T.item0 + li;
         ++k;
-        cc = cursor_next(cc, sc, gt, st, ntiles, rev);
+        cursor_next(cc, sc, st, ntiles, rev);
     }
     __syncthreads();
     if (warp < kNComp) store_item_comp(red[(k - 1) & 1], warp, part, nitems, prev);
