@@ -33,11 +33,13 @@
  *
  * What bounds it (967 x 967, 144 blocks of 7 x 1 items, 11.0 k cycles =
  * 5.5 us per iteration; k_solve took 25 us): the second half 5.0 k, bound by
- * instruction issue (about 300 warp instructions per item, 80 of them register
- * moves and addresses, and 20 FP32-to-FP64 conversions at a quarter of the
- * issue rate); the exchange 2.5 k from the last store to the totals, of which
- * 1.3 k are the least that one store and one load of a line another SM has
- * just written take; the first half 1.3 k, sending 1.2 k, the scalars 0.6 k.
+ * no single pipe (290 warp instructions per item in both halves, 20 of them
+ * FP32-to-FP64 conversions at a quarter of the issue rate, and 33 of the
+ * load-store unit; FP32 dots would take 3.8 k, neighbours by shuffle 6.1 k,
+ * and asking for the next item's tensor-memory words ahead changes nothing);
+ * the exchange 2.5 k from the last store to the totals, of which 1.3 k are the
+ * least that one store and one load of a line another SM has just written
+ * take; the first half 1.3 k, sending 1.2 k, the scalars 0.6 k.
  * Regions instead of items dealt out by the slots of k_solve's reduction tree
  * cut the rims of this tile from 1280 to 352 pixels per block and use all
  * SMs, and one FP64 sum per thread replaces a warp tree per item over FP32

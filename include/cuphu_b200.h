@@ -275,7 +275,9 @@ int cuphu_laplace_solve_device(const void *d_costs, int cost_stride_shorts,
  * job-size class (floor(log2) of the arc or work-item count) for all later
  * calls.  choices (optional, int[2]) receives {cost variant 0|1, solver
  * shape index}.  Results are identical for every choice: the per-item and
- * per-tile reductions do not depend on the launch shape.  CUPHU_TUNE=0 in
+ * per-tile reductions do not depend on the launch shape.  The shape is that
+ * of the solver that streams a tile's state; where all tiles of the probe stay
+ * on the chip, which has one shape, it is not stored.  CUPHU_TUNE=0 in
  * the environment ignores stored choices. */
 int cuphu_autotune(const float *igram_c64, const float *corr, int nrow, int ncol,
                    CuPhuCostMode cost_mode, const CuPhuParams *params,
@@ -444,7 +446,7 @@ int cuphu_gpu_info(int device, long long *total_memory, int *sm_count, int *cc_m
                    int *cc_minor);
 
 /* test hook (new): the next persistent solve launched on gpu_id runs with
- * block `block` not arriving at its first grid barrier, so every block's
+ * block `block` not arriving at its first barrier, so every block's
  * bounded wait runs out after CuPhuSolveOptions.timeout_ms and the call's
  * device status becomes CUPHU_ERR_TIMEOUT (read by cuphu_last_status, or
  * returned by calls that wait).  One-shot: later launches are normal. */
