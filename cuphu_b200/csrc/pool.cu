@@ -32,12 +32,14 @@ cudaMemPool_t pool_of(int dev)
         props.location.id = dev;
         cudaMemPool_t p = nullptr;
         unsigned long long keep = kPoolKeep;
-        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
-            cudaGetLastError();
+        /* the first use may lie inside a stream capture, of this thread or another, which a call
+         * that is not stream-ordered would invalidate; making a pool touches no stream */
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        const bool relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) p = nullptr;
+        if (p) cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
+        cudaGetLastError();
         g_pool[dev] = p;
     }
     return g_pool[dev];
