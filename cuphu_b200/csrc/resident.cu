@@ -579,6 +579,7 @@ __device__ __noinline__ int iterate()
             sh.active = act;
             sh.k = k;
             sh.seq = seq;
+            if ((k & 7) == 0 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
         }
         __syncthreads();
         if (!sh.active) return kStop;
@@ -605,7 +606,6 @@ __device__ __noinline__ int iterate()
         if (!__syncthreads_and(ok)) return kGaveUp;
         half2(C, ++seq);
         fresh = false;
-        if ((k & 63) == 63 && threadIdx.x == 0 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
     }
 }
 

@@ -158,7 +158,10 @@ __device__ __forceinline__ bool poll_together(ResShared &sh, There there)
  * barrier number n is passed at n x (blocks of the group).  With
  * `any_progress` the wait may outlast the limit as long as some block of
  * the launch still finishes exchanges (a block that is free early waits here for
- * partners that are still in an earlier tile). */
+ * partners that are still in an earlier tile).  Every running tile counts its
+ * progress up after each eighth iteration, whatever follows it, so the limit
+ * only has to cover eight iterations with their residual replacements (0.3 ms
+ * for tiles of 1000 x 1000 pixels, two side by side). */
 __device__ __noinline__ bool group_sync(bool any_progress = false)
 {
     ResShared &sh = res_shared();

@@ -687,7 +687,7 @@ __device__ __noinline__ bool iterate()
                 sh.beta = quotient_pos(tot, S.rz);
                 S.rz = tot;
             }
-            if ((it & 63) == 63 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
+            if ((it & 7) == 0 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
         }
         __syncthreads();
         if (!sh.active) break;

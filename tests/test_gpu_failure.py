@@ -10,7 +10,7 @@ import pytest
 
 import oracle as O
 from cuphu_b200 import synthetic as S
-from cuphu_b200._lib import (CuPhuError, CuPhuSolveStats, check, default_params,
+from cuphu_b200._lib import (CuPhuError, CuPhuScene, CuPhuSolveStats, check, default_params,
                              default_solve_options, default_tile_params, lib)
 from tests.devbuf import dptr, empty, to_dev, to_host
 
@@ -57,3 +57,27 @@ def test_skipped_barrier_times_out_and_device_recovers(torch_cuda, precision):
     check(rc)
     assert lib().cuphu_last_status(0) == 0
     assert np.array_equal(got.view(np.int32), want.view(np.int32))
+
+
+@pytest.mark.parametrize("precision,replace,side", [(0, 1, 1000), (0, 50, 1000), (1, 0, 700)])
+def test_waiting_for_another_tile_is_not_a_timeout(torch_cuda, precision, replace, side):
+    """Three equal scenes of which two run side by side: the remaining blocks wait for the third
+    scene's partners far longer than the limit (about 15 ms with a replacement in every
+    iteration), but those make progress, so the call succeeds."""
+    scenes = (CuPhuScene * 3)()
+    keep = []
+    for i in range(3):
+        ig, g, _, _ = S.bumps(side, side, seed=9 + i, nbumps=3, amp_range=(20, 40),
+                              sigma_range=(30, 90))
+        ph = np.mod(np.angle(ig), 2 * np.pi).astype(np.float32)
+        bufs = (to_dev(ph), to_dev(g), empty((side, side), torch_cuda.float32),
+                empty((side, side), torch_cuda.int32))
+        keep.append(bufs)
+        scenes[i] = CuPhuScene(None, bufs[0].data_ptr(), bufs[1].data_ptr(), None, None, side,
+                               side, 1, 1, 0, 0, 5.0, bufs[2].data_ptr(), bufs[3].data_ptr())
+    p = default_params()
+    o = default_solve_options(precision=precision, n_irls=0, max_iter=400, timeout_ms=5,
+                              replace_every=replace)
+    st = CuPhuSolveStats()
+    check(lib().cuphu_unwrap_batch_device(scenes, 3, 0, C.byref(p), C.byref(o), C.byref(st), None))
+    assert st.total_iters == 400
