@@ -25,8 +25,10 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
+#include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -82,6 +84,21 @@ int host_threads()
     return (int)std::max(1u, std::min(hc, 64u));
 }
 
+/* Up to n threads that run work(), which takes chunks until none is left; fewer
+ * where the system starts no more (a limit on threads or memory), and where it
+ * starts none the caller does the work here. */
+template <typename Work> std::vector<std::thread> start_workers(int n, const Work &work)
+{
+    std::vector<std::thread> pool;
+    pool.reserve(n);
+    try {
+        for (int t = 0; t < n; ++t) pool.emplace_back(std::cref(work));
+    } catch (const std::system_error &) {
+        if (pool.empty()) work();
+    }
+    return pool;
+}
+
 }  // namespace
 
 static size_t chunk_of(size_t n)
@@ -99,17 +116,14 @@ void compute_host_phase(const float *c64, const float *re, const float *im, size
         return;
     }
     std::atomic<size_t> next(0);
-    std::vector<std::thread> pool;
-    pool.reserve(nth);
-    for (int t = 0; t < nth; ++t)
-        pool.emplace_back([&]() {
-            for (;;) {
-                size_t c = next.fetch_add(1, std::memory_order_relaxed);
-                if (c >= nch) return;
-                phase_range(c64, re, im, out, c * chunk, std::min(n, (c + 1) * chunk));
-            }
-        });
-    for (auto &th : pool) th.join();
+    const auto work = [&]() {
+        for (;;) {
+            size_t c = next.fetch_add(1, std::memory_order_relaxed);
+            if (c >= nch) return;
+            phase_range(c64, re, im, out, c * chunk, std::min(n, (c + 1) * chunk));
+        }
+    };
+    for (auto &th : start_workers(nth, work)) th.join();
 }
 
 int upload_host_phase(const float *c64, const float *re, const float *im, size_t n, float *d_ph,
@@ -150,18 +164,16 @@ int upload_host_phase(const float *c64, const float *re, const float *im, size_t
         std::unique_ptr<std::atomic<int>[]> ready(new std::atomic<int>[nch]);
         for (size_t c = 0; c < nch; ++c) ready[c].store(0, std::memory_order_relaxed);
         std::atomic<size_t> next(0);
-        std::vector<std::thread> pool;
-        pool.reserve(nth);
-        for (int t = 0; t < nth; ++t)
-            pool.emplace_back([&]() {
-                for (;;) {
-                    size_t c = next.fetch_add(1, std::memory_order_relaxed);
-                    if (c >= nch) return;
-                    size_t a = c * chunk, b = std::min(n, a + chunk);
-                    phase_range(c64, re, im, P.buf, a, b);
-                    ready[c].store(1, std::memory_order_release);
-                }
-            });
+        const auto work = [&]() {
+            for (;;) {
+                size_t c = next.fetch_add(1, std::memory_order_relaxed);
+                if (c >= nch) return;
+                size_t a = c * chunk, b = std::min(n, a + chunk);
+                phase_range(c64, re, im, P.buf, a, b);
+                ready[c].store(1, std::memory_order_release);
+            }
+        };
+        std::vector<std::thread> pool = start_workers(nth, work);
         for (size_t c = 0; c < nch; ++c) {
             while (!ready[c].load(std::memory_order_acquire)) std::this_thread::yield();
             if (rc) continue;
