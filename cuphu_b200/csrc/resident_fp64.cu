@@ -29,6 +29,7 @@
  * halves.  Per iteration 5.5 us at 256 x 256, 6.2 us at 512 x 512, 11.1 us at
  * 967 x 967; the streaming form took 22, 28 and 50 us.
  */
+#include "quotient.cuh"
 #include "resident_geom.cuh"
 
 namespace cuphu {
@@ -156,48 +157,6 @@ __device__ __forceinline__ void lds2(const double *p, double v[2])
 __device__ __forceinline__ void sts2(double *p, const double v[2])
 {
     *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
-}
-
-/* r / d from y = RN(1/d).  The correction steps are exact where nothing
- * underflows or overflows: for a residual that is zero or in [2^-900, 2^900]
- * (res_odd tests the rest) and a diagonal in [2^-100, 2^100] (y = 0 marks the
- * rest).  A block that meets another value forms its quotients with IEEE
- * divisions, in functions of their own (slow_fold, slow_update): a division
- * in the iterations would be a call there, and cost them their registers. */
-__device__ __forceinline__ double quotient(double r, double d, double y)
-{
-    const double q0 = __dmul_rn(r, y);
-    const double q1 = __fma_rn(__fma_rn(-q0, d, r), y, q0);
-    return __fma_rn(__fma_rn(-q1, d, r), y, q1);
-}
-__device__ __forceinline__ bool res_odd(double r)
-{
-    const unsigned e = ((unsigned)__double2hiint(r) & 0x7fffffffu) - (123u << 20);
-    return e > (1800u << 20) && r != 0.0;
-}
-
-/* a / b rounded to nearest for a, b > 0, without the call that the division
- * operator can make (a call in the iterations would push q = A p out of the
- * registers): the reciprocal by Newton steps from the hardware's
- * approximation, then Markstein's two correction steps.  Operands outside
- * [2^-900, 2^900] are scaled by 2^+-600 first; a result that is not a normal
- * number may differ from the operator's in its last bit. */
-__device__ __forceinline__ double quotient_pos(double a, double b)
-{
-    auto scale = [](double v) {
-        const int e = (__double2hiint(v) >> 20) & 0x7ff;
-        return e < 123 ? 0x1p600 : e > 1923 ? 0x1p-600 : 1.0;
-    };
-    const double sa = scale(a), sb = scale(b);
-    a *= sa;
-    b *= sb;
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
-    const double q = quotient(a, b, y);
-    const double back = sa == 1.0 ? 1.0 : sa > 1.0 ? 0x1p-600 : 0x1p600;   /* 1 / sa */
-    return (q * back) * sb;
 }
 
 /* A block's mailbox: [parity][member m] packets, four copies of each (64
@@ -627,7 +586,7 @@ __device__ __noinline__ bool iterate()
         if (!total(C, seq, tot)) return false;
         if (threadIdx.x == 0) {
             if (tot <= 0.0) sh.active = 0;
-            else sh.alpha = quotient_pos(S.rz, tot);
+            else sh.alpha = quotient_any(S.rz, tot);
         }
         __syncthreads();
         if (!sh.active) break;
@@ -684,7 +643,7 @@ __device__ __noinline__ bool iterate()
             if (tot < S.thr || it >= sh.K.sp.max_iter) {
                 sh.active = 0;
             } else {
-                sh.beta = quotient_pos(tot, S.rz);
+                sh.beta = quotient_any(tot, S.rz);
                 S.rz = tot;
             }
             if ((it & 7) == 0 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
