@@ -579,8 +579,9 @@ __device__ __noinline__ int iterate()
             sh.active = act;
             sh.k = k;
             sh.seq = seq;
-            if ((k & 7) == 0 && sh.member == 0) atomicAdd(&sh.K.ctl->progress, 1u);
         }
+        if (threadIdx.x == kResThreads - 1 && (k & 7) == 0 && sh.member == 0)
+            atomicAdd(&sh.K.ctl->progress, 1u);   /* while thread 0 forms the scalars */
         __syncthreads();
         if (!sh.active) return kStop;
         if (sp.replace_every > 0 && k % sp.replace_every == 0) return kReplace;
