@@ -151,6 +151,7 @@ SIGNATURES = {
     "cuphu_bridge_device": (_I, [VP, VP, VP, _I, _I, P(CuPhuBridgeParams), VP]),
     "cuphu_test_skip_barrier_once": (_I, [_I, _I]),
     "cuphu_test_force_solve_shape": (_I, [_I]),
+    "cuphu_test_solver_plan": (_I, [P(_I), P(_I), _I, _I, _I, P(_I)]),
     "cuphu_last_status": (_I, [_I]),
     "cuphu_release_workspace": (_I, [_I]),
 }

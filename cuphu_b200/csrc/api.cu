@@ -1917,6 +1917,27 @@ int cuphu_gpu_info(int device, long long *total_memory, int *sm_count, int *cc_m
     return 0;
 }
 
+int cuphu_test_solver_plan(const int *nrow, const int *ncol, int ntiles, int sm_count,
+                           int precision, int *out)
+{
+    if (!nrow || !ncol || !out || ntiles < 1 || sm_count < 1)
+        return fail(CUPHU_ERR_INVALID, "bad arguments");
+    std::vector<TileDesc> tiles(ntiles);
+    for (int t = 0; t < ntiles; ++t) {
+        if (nrow[t] < 1 || ncol[t] < 1) return fail(CUPHU_ERR_INVALID, "bad tile");
+        tiles[t].nbx = (ncol[t] + kItemBx - 1) / kItemBx;
+        tiles[t].nitems = tiles[t].nbx * ((nrow[t] + kItemBy - 1) / kItemBy);
+    }
+    ResidentPlan plan;
+    plan_resident(tiles, sm_count, precision == CUPHU_PREC_FP64, plan);
+    std::fill(out, out + 4 * (size_t)ntiles, 0);
+    for (const ResTile &R : plan.sched) {
+        const int v[4] = {1, R.nact, R.a, R.b};
+        std::copy(v, v + 4, out + 4 * (size_t)R.tile);
+    }
+    return plan.nblk;
+}
+
 int cuphu_last_status(int gpu_id)
 {
     if (gpu_id < 0 || gpu_id >= 64) return fail(CUPHU_ERR_INVALID, "device index out of range");

@@ -458,6 +458,14 @@ int cuphu_test_skip_barrier_once(int gpu_id, int block);
  * overriding stored autotuner choices; -1 restores the normal choice. */
 int cuphu_test_force_solve_shape(int shape);
 
+/* test hook (new): how the solver would split a job of `ntiles` tiles (rows x
+ * columns) on a GPU of sm_count SMs, without using one.  Four numbers per
+ * tile: 1 if its state is kept on the chip (0: streamed, the rest zero), the
+ * blocks of its group, and in mixed precision the rows and columns of a
+ * block's region in items of 16 x 64 pixels.  Returns the blocks launched. */
+int cuphu_test_solver_plan(const int *nrow, const int *ncol, int ntiles, int sm_count,
+                           int precision, int *out);
+
 /* wait for the last pipeline enqueued on a device and return its device-side
  * status (CUPHU_ERR_TIMEOUT when a grid barrier gave up) (new) */
 int cuphu_last_status(int gpu_id);
