@@ -367,9 +367,13 @@ struct SolverJob {
         sp.skip_block = solver_take_skip_block(dev);
         sp.pass_iters = d_pass;
         int rc = 0;
-        if (res.nblk)
-            rc = fp64 ? launch_resident_fp64(res, d_tiles, P, d_ctl, sp, s)
-                      : launch_resident_mixed(res, d_tiles, P, d_ctl, sp, s);
+        if (res.nblk) {
+            SolveParams on_chip = sp;
+            /* every launched block has work: a plan takes the lowest free ones */
+            if (sp.skip_block >= 0) on_chip.skip_block = sp.skip_block % res.nblk;
+            rc = fp64 ? launch_resident_fp64(res, d_tiles, P, d_ctl, on_chip, s)
+                      : launch_resident_mixed(res, d_tiles, P, d_ctl, on_chip, s);
+        }
         if (!rc && !stream.empty())
             rc = launch_solve(fp64, d_stream, d_item, stream_items, (int)stream.size(), P, pitch,
                               rows, d_st, d_part, d_ctl, sp, dev, s);

@@ -1614,7 +1614,7 @@ static int make_maps(SolveMaps &M, const SolverPlanes &P, int pitch, int rows)
 template <typename V, bool WLS, int NS, int MINB>
 static int launch_solve_shape(const TileDesc *tiles, const int *item_tile, int nitems,
                               int ntiles, const SolverPlanes &P, int pitch, int rows,
-                              TileState *st, double *part, SolverCtl *ctl, const SolveParams &sp,
+                              TileState *st, double *part, SolverCtl *ctl, SolveParams sp,
                               long long timeout_ns, int device, cudaStream_t s)
 {
     SolveMaps M;
@@ -1632,6 +1632,7 @@ static int launch_solve_shape(const TileDesc *tiles, const int *item_tile, int n
     if (per_sm < 1) return fail(CUPHU_ERR_CUDA, "solver kernel cannot be resident");
     per_sm = std::min(per_sm, MINB);
     int grid = std::min(nsm * per_sm, std::max(nitems, 1));
+    if (sp.skip_block >= 0) sp.skip_block %= grid;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kItemThreads);

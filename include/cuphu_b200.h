@@ -446,10 +446,11 @@ int cuphu_gpu_info(int device, long long *total_memory, int *sm_count, int *cc_m
                    int *cc_minor);
 
 /* test hook (new): the next persistent solve launched on gpu_id runs with
- * block `block` not arriving at its first barrier, so every block's
- * bounded wait runs out after CuPhuSolveOptions.timeout_ms and the call's
- * device status becomes CUPHU_ERR_TIMEOUT (read by cuphu_last_status, or
- * returned by calls that wait).  One-shot: later launches are normal. */
+ * block `block` (modulo the blocks of the launch) not arriving at its first
+ * barrier, so the bounded waits of the blocks it works with run out after
+ * CuPhuSolveOptions.timeout_ms and the call's device status becomes
+ * CUPHU_ERR_TIMEOUT (read by cuphu_last_status, or returned by calls that
+ * wait).  One-shot: later launches are normal. */
 int cuphu_test_skip_barrier_once(int gpu_id, int block);
 
 /* test hook (new): solves launched later from the calling thread use launch

@@ -81,3 +81,17 @@ def test_waiting_for_another_tile_is_not_a_timeout(torch_cuda, precision, replac
     st = CuPhuSolveStats()
     check(lib().cuphu_unwrap_batch_device(scenes, 3, 0, C.byref(p), C.byref(o), C.byref(st), None))
     assert st.total_iters == 400
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("block", [0, 2, 40, 147, 100000])
+def test_skipped_barrier_of_any_block_number(torch_cuda, precision, block):
+    """A small scene's solve launches a few blocks; a number beyond them is taken modulo their
+    number, so the hook always does what it says."""
+    ig, g, _, _ = S.bumps(70, 90, seed=52, nbumps=2)
+    ph = O.phase_from_igram(ig)
+    check(lib().cuphu_test_skip_barrier_once(0, block))
+    rc, _ = _run(torch_cuda, ph, g, precision, 20, stats=True)
+    assert rc == TIMEOUT
+    rc, _ = _run(torch_cuda, ph, g, precision, 5000, stats=True)
+    check(rc)
