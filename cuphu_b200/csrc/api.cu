@@ -354,7 +354,6 @@ struct SolverJob {
     ResidentArgs res;                  /* device copies of the plan, and scratch */
     std::vector<TileDesc> stream;      /* the streamed tiles, items renumbered */
     const TileDesc *d_tiles = nullptr, *d_stream = nullptr;
-    const int *d_item = nullptr;
     int stream_items = 0;
     TileState *d_st = nullptr;
     double *d_part = nullptr;
@@ -375,8 +374,8 @@ struct SolverJob {
                       : launch_resident_mixed(res, d_tiles, P, d_ctl, on_chip, s);
         }
         if (!rc && !stream.empty())
-            rc = launch_solve(fp64, d_stream, d_item, stream_items, (int)stream.size(), P, pitch,
-                              rows, d_st, d_part, d_ctl, sp, dev, s);
+            rc = launch_solve(fp64, d_stream, stream_items, (int)stream.size(), P, pitch, rows, d_st,
+                              d_part, d_ctl, sp, dev, s);
         return rc;
     }
     /* iteration statistics, after the launches are complete */
@@ -683,7 +682,6 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     SJ.res.nblk = SJ.plan.nblk;
     SJ.d_tiles = d_tiles;
     SJ.d_stream = d_stream;
-    SJ.d_item = d_item;
     SJ.d_st = d_st;
     SJ.d_part = d_part;
     SJ.d_ctl = d_ctl;

@@ -136,10 +136,9 @@ int upload_host_phase(const float *c64, const float *re, const float *im, size_t
 void compute_host_phase(const float *c64, const float *re, const float *im, size_t n, float *out);
 
 /* laplace.cu */
-int launch_solve(bool fp64, const TileDesc *tiles, const int *item_tile, int nitems,
-                 int ntiles, const SolverPlanes &P, int plane_pitch, int plane_rows,
-                 TileState *st, double *part, SolverCtl *ctl, const SolveParams &sp,
-                 int device, cudaStream_t s);
+int launch_solve(bool fp64, const TileDesc *tiles, int nitems, int ntiles, const SolverPlanes &P,
+                 int plane_pitch, int plane_rows, TileState *st, double *part, SolverCtl *ctl,
+                 const SolveParams &sp, int device, cudaStream_t s);
 /* the solver's launch shapes (ring stages, blocks per SM) the autotuner
  * chooses among, per precision; shape v of solve_shape_count(fp64) */
 int solve_shape_count(bool fp64);

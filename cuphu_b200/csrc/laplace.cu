@@ -1266,9 +1266,9 @@ __device__ __forceinline__ void carry_inactive(const TileState *from, TileState 
  * main path's register allocation does not carry its extra inputs */
 template <typename V, bool WLS, int NS, int MINB>
 __global__ void __launch_bounds__(kItemThreads, MINB)
-    k_solve(const TileDesc *__restrict__ tiles, const int *__restrict__ item_tile, int nitems,
-            int ntiles, SolverPlanes P, TileState *st, double *part, SolverCtl *ctl,
-            SolveParams sp, long long timeout_ns, const __grid_constant__ SolveMaps M)
+    k_solve(const TileDesc *__restrict__ tiles, int nitems, int ntiles, SolverPlanes P,
+            TileState *st, double *part, SolverCtl *ctl, SolveParams sp, long long timeout_ns,
+            const __grid_constant__ SolveMaps M)
 {
     extern __shared__ __align__(128) char dsm_raw[];
     __shared__ double sw[32];
@@ -1294,7 +1294,6 @@ __global__ void __launch_bounds__(kItemThreads, MINB)
      * buffered in the z and r planes */
     V *zb[2] = {(V *)P.z, (V *)P.r};
     uint32_t parity = 0u;   /* phase bit per stage of the ring */
-    (void)item_tile;
     if (threadIdx.x == 0) {
         for (int k = 0; k < NS; ++k) mbar_init(&bars[k]);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1612,8 +1611,8 @@ static int make_maps(SolveMaps &M, const SolverPlanes &P, int pitch, int rows)
  * depend on the shape, so every shape gives identical results; the
  * autotuner times them and keeps the fastest per job size. */
 template <typename V, bool WLS, int NS, int MINB>
-static int launch_solve_shape(const TileDesc *tiles, const int *item_tile, int nitems,
-                              int ntiles, const SolverPlanes &P, int pitch, int rows,
+static int launch_solve_shape(const TileDesc *tiles, int nitems, int ntiles,
+                              const SolverPlanes &P, int pitch, int rows,
                               TileState *st, double *part, SolverCtl *ctl, SolveParams sp,
                               long long timeout_ns, int device, cudaStream_t s)
 {
@@ -1643,13 +1642,13 @@ static int launch_solve_shape(const TileDesc *tiles, const int *item_tile, int n
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CUPHU_TRY_CUDA(cudaLaunchKernelEx(&cfg, kern, tiles, item_tile, nitems, ntiles, P, st, part,
+    CUPHU_TRY_CUDA(cudaLaunchKernelEx(&cfg, kern, tiles, nitems, ntiles, P, st, part,
                                       ctl, sp, timeout_ns, M));
     return 0;
 }
 
 template <typename V, bool WLS>
-static int launch_solve_kernel(const TileDesc *tiles, const int *item_tile, int nitems, int ntiles,
+static int launch_solve_kernel(const TileDesc *tiles, int nitems, int ntiles,
                           const SolverPlanes &P, int pitch, int rows, TileState *st, double *part,
                           SolverCtl *ctl, const SolveParams &sp, long long timeout_ns, int device,
                           cudaStream_t s)
@@ -1660,7 +1659,7 @@ static int launch_solve_kernel(const TileDesc *tiles, const int *item_tile, int 
     tune_note_items(nitems);
     const int v = tune_get(device, sizeof(V) == 8 ? 2 : 1, (long long)nitems);
 #define CUPHU_SOLVE_SHAPE(NS, MINB)                                                            \
-    return launch_solve_shape<V, WLS, NS, MINB>(tiles, item_tile, nitems, ntiles, P, pitch,    \
+    return launch_solve_shape<V, WLS, NS, MINB>(tiles, nitems, ntiles, P, pitch,    \
                                                 rows, st, part, ctl, sp, timeout_ns, device, s)
     if constexpr (sizeof(V) == 4) {
         switch (v) {
@@ -1691,15 +1690,15 @@ void solve_shape_of(bool fp64, int v, int *stages, int *blocks_per_sm)
 }
 
 template <typename V>
-static int launch_solve_t(const TileDesc *tiles, const int *item_tile, int nitems, int ntiles,
+static int launch_solve_t(const TileDesc *tiles, int nitems, int ntiles,
                           const SolverPlanes &P, int pitch, int rows, TileState *st, double *part,
                           SolverCtl *ctl, const SolveParams &sp, long long timeout_ns, int device,
                           cudaStream_t s)
 {
     if (sp.wls)
-        return launch_solve_kernel<V, true>(tiles, item_tile, nitems, ntiles, P, pitch, rows, st,
+        return launch_solve_kernel<V, true>(tiles, nitems, ntiles, P, pitch, rows, st,
                                             part, ctl, sp, timeout_ns, device, s);
-    return launch_solve_kernel<V, false>(tiles, item_tile, nitems, ntiles, P, pitch, rows, st, part,
+    return launch_solve_kernel<V, false>(tiles, nitems, ntiles, P, pitch, rows, st, part,
                                          ctl, sp, timeout_ns, device, s);
 }
 
@@ -1719,16 +1718,16 @@ int solver_take_skip_block(int dev)
     return dev >= 0 && dev < 64 ? g_skip_block[dev].exchange(-1) : -1;
 }
 
-int launch_solve(bool fp64, const TileDesc *tiles, const int *item_tile, int nitems,
-                 int ntiles, const SolverPlanes &P, int plane_pitch, int plane_rows,
+int launch_solve(bool fp64, const TileDesc *tiles, int nitems, int ntiles,
+                 const SolverPlanes &P, int plane_pitch, int plane_rows,
                  TileState *st, double *part, SolverCtl *ctl, const SolveParams &sp,
                  int device, cudaStream_t s)
 {
     long long timeout_ns = sp.timeout_ns;
     if (fp64)
-        return launch_solve_t<double>(tiles, item_tile, nitems, ntiles, P, plane_pitch, plane_rows,
+        return launch_solve_t<double>(tiles, nitems, ntiles, P, plane_pitch, plane_rows,
                                       st, part, ctl, sp, timeout_ns, device, s);
-    return launch_solve_t<float>(tiles, item_tile, nitems, ntiles, P, plane_pitch, plane_rows, st,
+    return launch_solve_t<float>(tiles, nitems, ntiles, P, plane_pitch, plane_rows, st,
                                  part, ctl, sp, timeout_ns, device, s);
 }
 
