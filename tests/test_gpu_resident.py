@@ -120,3 +120,23 @@ def test_fp64_division_outside_the_correction_range(torch_cuda):
            for e in (60, 120)]
     assert t.isfinite(out[0]).all() and float(out[0].abs().max()) > 0
     assert t.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("tiny", [-930, -980])
+def test_fp64_residuals_outside_the_correction_range(torch_cuda, tiny):
+    """A warm start of one pixel of 1 and, far from it, one of 2^tiny, without targets: residuals
+    of the second lie below the range of the correction steps and take the IEEE division.  The
+    same scaled by 2^150 stays inside the range; the problem is linear, so the solutions agree bit
+    for bit."""
+    from cuphu_b200.autograd import wls_solve
+    t = torch_cuda
+    g = t.Generator(device="cuda")
+    g.manual_seed(4)
+    wd, wr = (t.rand((100, 140), generator=g, device="cuda") + 0.5 for _ in range(2))
+    none = t.zeros_like(wd)
+    u0 = t.zeros((100, 140), dtype=t.float64, device="cuda")
+    u0[20, 20], u0[70, 110] = 1.0, 2.0 ** tiny
+    out = [wls_solve(none, none, wd, wr, u0=u0 * s, max_iter=20) / s for s in (1.0, 2.0 ** 150)]
+    assert 0.0 < float(out[0][70, 110]) < 2.0 ** tiny
+    assert float(out[0][71, 110]) > 0.0
+    assert t.equal(out[0], out[1])
