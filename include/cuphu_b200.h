@@ -194,8 +194,14 @@ int cuphu_unwrap_device(const float *igram_c64, const float *phase_in, const flo
                         uint32_t *conncomp_out, int32_t *cycles_out,
                         CuPhuSolveStats *stats, void *stream);
 
-/* new: batched solve of many independent scenes in one persistent launch
- * (device pointers; tiles of every scene share one solver launch). */
+/* new: batched solve of many independent scenes in one job (device pointers;
+ * the tiles of all scenes share one launch of the solver that keeps a tile's
+ * state on the chip and one of the solver that streams it).  In FP64 a
+ * scene's results are those of its own call, bit for bit.  In mixed precision
+ * the split of an on-chip tile over the GPU, and with it the order in which
+ * its FP64 dot products are summed, depends on the job: the sums agree to
+ * about 1e-14, so that results are equal as a rule, but a last bit of the
+ * solution, and at a pixel near a half cycle its cycle, may differ. */
 typedef struct CuPhuScene {
     const float         *igram_c64;   /* device, or NULL with phase      */
     const float         *phase;       /* device wrapped phase, or NULL   */
@@ -471,7 +477,10 @@ int cuphu_test_solver_plan(const int *nrow, const int *ncol, int ntiles, int sm_
  * status (CUPHU_ERR_TIMEOUT when a grid barrier gave up) (new) */
 int cuphu_last_status(int gpu_id);
 
-/* release the cached per-device workspace (new) */
+/* release the cached per-device workspace and the memory that the library's
+ * pool holds for its scratch allocations (at most 1 GiB per device stay with
+ * it across synchronisations; the process's own allocations take them back
+ * when the GPU has no other memory left) (new) */
 int cuphu_release_workspace(int gpu_id);
 
 #ifdef __cplusplus
