@@ -41,14 +41,24 @@ FALLBACK_HBM = 6650.0
 METRIC = "Mpix/s unwrapped at 8192^2 (mixed-precision Laplace PCG)"
 
 
-# measured k_resident DRAM bytes (mixed precision), see the roofline block:
-# ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4096^2 case (4 x 4
-# tiles, 18.39 M tile pixels): 618.6 MB for one pass of 20 iterations, 619.1
-# for 60, 950.9 for three passes of 20, 620.2 with six residual replacements.
-# Nothing crosses the HBM between iterations; the first pass of a tile reads
-# and writes its planes, the later ones find most of them in the L2
+# the solver kernels' measured work, see the roofline block.  On-chip solvers:
+# ncu smsp__inst_executed.sum of one 967^2 tile at 300 iterations less that at
+# 100, per warp and 16 x 64-pixel work item and iteration (mixed, FP64)
+INST_PER_WARP_ITEM = (291, 464)
+# and ncu dram__bytes_read.sum + dram__bytes_write.sum of the mixed 4096^2 case
+# (4 x 4 tiles, 18.39 M tile pixels): 618.6 MB for one pass of 20 iterations,
+# 619.1 for 60, 950.9 for three passes of 20, 620.2 with six residual
+# replacements.  Nothing crosses the HBM between iterations; the first pass of a
+# tile reads and writes its planes, the later ones find most of them in the L2
 TRAFFIC_FIRST_PASS_PX = 33.6
 TRAFFIC_PER_PASS_PX = 9.0
+# streaming solver (mixed), the same case when it ran the tiles, at 20, 40 and
+# 60 iterations of one pass: 17.84, 33.80 and 50.52 GB.  40 - 20: bytes per
+# pixel-iteration; the intercept: per tile pixel of a pass; 60 - 40 beyond 20
+# iterations: the one true-residual replacement
+STREAM_PER_PX_ITER = 43.4
+STREAM_PER_PASS_PX = 102.3
+STREAM_PER_REPL_PX = 40.8
 
 
 def hbm_peak():
@@ -57,6 +67,53 @@ def hbm_peak():
             return float(json.load(f)["hbm_gbs"]), "measured"
     except Exception:
         return FALLBACK_HBM, "fallback"
+
+
+def solver_roofline(tiles, prec, opts, st, sm_count, clk):
+    """Roofline of the dominant kernel, the Laplace solve, which depends on where the tiles' state
+    lies.  On the chip: bound by instruction issue, so the warp instructions of the iterations
+    (pixels of the active tiles only, no padding) per second against four per SM and cycle; what is
+    missing is the exchange between the blocks, the scalars and idle blocks.  Streamed: bound by
+    HBM, so tile pixels x (36 B (FP64 64) per PCG iteration x iterations of the active tiles + 38 B
+    per IRLS pass for assembly and reweight + 12 B per true-residual replacement, one SpMV read of x
+    and the weights)."""
+    from cuphu_b200._lib import check, lib
+    n = len(tiles)
+    ip, plan = C.POINTER(C.c_int), (C.c_int * (4 * n))()
+    rows, cols = ((C.c_int * n)(*[t[k] for t in tiles]) for k in (0, 1))
+    check(min(0, lib().cuphu_test_solver_plan(rows, cols, n, sm_count, prec, C.cast(plan, ip))))
+    kept = sum(plan[4 * t] for t in range(n))
+    tile_px = sum(r * c for r, c in tiles)
+    px_iters = st.px_iters                # iterations x pixels of the active tiles
+    seconds = st.solve_ms * 1e-3
+    passes = opts.n_irls + 1
+    # pixels of the replacements: every tile replaces its residual once per
+    # replace_every of its iterations (mixed precision only)
+    repl_px = px_iters / opts.replace_every if prec == 0 and opts.replace_every > 0 else 0.0
+    streaming = (px_iters * (36 if prec == 0 else 64) + passes * tile_px * 38 + repl_px * 12)
+    hbm, hbm_kind = hbm_peak()
+    out = {"solve_ms": st.solve_ms, "pcg_iterations": st.total_iters, "px_iterations": px_iters,
+           "tile_px": tile_px, "tiles_on_chip": kept, "tiles_streamed": n - kept,
+           "hbm_gbs_if_streamed": streaming / seconds / 1e9}
+    if kept == n:
+        mhz = clk["sm_mhz"] if clk and clk.get("sm_mhz") else 1965.0
+        inst = px_iters * INST_PER_WARP_ITEM[prec] * 8 / 1024.0
+        achieved, peak = inst / seconds / 1e9, sm_count * 4 * mhz / 1e3
+        out.update(kernel="k_resident" if prec == 0 else "k_resident64", bound="instruction issue",
+                   achieved=achieved, peak=peak, unit="G warp instructions/s",
+                   frac=achieved / peak, peak_kind="4 per SM and cycle at the sampled clock",
+                   traffic=(tile_px * (TRAFFIC_FIRST_PASS_PX + opts.n_irls * TRAFFIC_PER_PASS_PX)
+                            if prec == 0 else None))
+    elif kept == 0:
+        out.update(kernel="k_solve", bound="hbm", achieved=streaming / seconds / 1e9, peak=hbm,
+                   unit="GB/s", frac=streaming / seconds / 1e9 / hbm, peak_kind=hbm_kind,
+                   traffic=(px_iters * STREAM_PER_PX_ITER + passes * tile_px * STREAM_PER_PASS_PX +
+                            repl_px * STREAM_PER_REPL_PX if prec == 0 else None))
+    else:
+        out.update(kernel=("k_resident" if prec == 0 else "k_resident64") + ", then k_solve",
+                   bound="two launches, not separated", achieved=None, peak=None, unit=None,
+                   frac=None, peak_kind=None, traffic=None)
+    return out
 
 
 class ClockSampler:
@@ -589,6 +646,7 @@ def run_reference(args, rank, world):
 
 def run_ours(args, rank, world, local_rank):
     import torch
+    import cuphu_b200
     from cuphu_b200.replicas import max_over_ranks
     from cuphu_b200._lib import (CuPhuSolveStats, check, default_params, default_solve_options,
                                  default_tile_params, lib)
@@ -680,35 +738,11 @@ def run_ours(args, rank, world, local_rank):
     step(opts, st)
     unw_mixed = d_u.cpu().numpy()
 
-    # roofline of the dominant kernel (the Laplace solve): the bytes of a
-    # solver that streams its state = tile pixels x (36 B per PCG iteration x
-    # iterations of the active tiles + 38 B per IRLS pass for assemble and
-    # reweight + 12 B per true-residual replacement, one SpMV read of x and
-    # the weights).  The tiles' state stays on the chip, so these bytes do not
-    # cross the HBM and the fraction may exceed one; `traffic` is what does
-    peak, peak_kind = hbm_peak()
     # tile extents of the reference's tile geometry (cuphu_solver.cpp:1753-1791)
     tr_f = [(int(t * (nrow - 64) / ntr), (nrow if t == ntr - 1 else int((t + 1) * (nrow - 64) / ntr) + 64)) for t in range(ntr)]
     tc_f = [(int(t * (ncol - 64) / ntc), (ncol if t == ntc - 1 else int((t + 1) * (ncol - 64) / ntc) + 64)) for t in range(ntc)]
-    tile_px = sum((b - a) for a, b in tr_f) * sum((b - a) for a, b in tc_f)
-    px_iters = st.px_iters                # iterations x pixels of the active tiles
-    bpi = 36 if prec == 0 else 64
-    # pixels of the replacements: every tile replaces its residual once per
-    # replace_every of its iterations (mixed precision only)
-    repl_px = px_iters / opts.replace_every if prec == 0 and opts.replace_every > 0 else 0.0
-    alg_bytes = px_iters * bpi + (opts.n_irls + 1) * tile_px * 38 + repl_px * 12
-    achieved = alg_bytes / (st.solve_ms * 1e-3) / 1e9
-    # DRAM traffic per launch, scaled from ncu captures of the 4096^2 case
-    traffic = (tile_px * (TRAFFIC_FIRST_PASS_PX + opts.n_irls * TRAFFIC_PER_PASS_PX)
-               if prec == 0 else None)
-    roofline = {"bound": "instruction issue and block exchange (state on chip)",
-                "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                "achieved_is": "bytes a solver streaming its state from HBM would move per second",
-                "kernel": "k_resident" if prec == 0 else "k_resident64",
-                "solve_ms": st.solve_ms, "pcg_iterations": st.total_iters,
-                "px_iterations": st.px_iters, "tile_px": tile_px,
-                "bytes_per_px_iter": bpi}
+    roofline = solver_roofline([(r1 - r0, c1 - c0) for r0, r1 in tr_f for c0, c1 in tc_f], prec,
+                               opts, st, cuphu_b200.gpu_info(local_rank)["sm_count"], clk)
 
     result = {}
     if rank == 0 and not args.skip_fp64 and prec == 0:
