@@ -804,7 +804,7 @@ def run_ours(args, rank, world, local_rank):
         cbytes = npix * 4 + npix * 4 + narcs * 8
         result["cost_build"] = {"kernel": "k_costs7<DEFO>", "ms": cms,
                                 "gbs": cbytes / (cms * 1e-3) / 1e9,
-                                "frac": cbytes / (cms * 1e-3) / 1e9 / peak,
+                                "frac": cbytes / (cms * 1e-3) / 1e9 / hbm_peak()[0],
                                 "bytes_per_px": cbytes / npix}
         del d_cost, d_ph
 
