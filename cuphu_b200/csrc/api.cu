@@ -484,6 +484,10 @@ static int run_job(std::vector<SceneIn> &S, const CuPhuParams &prm, const JobOpt
     plan_resident(pl.tiles, nsm, jo.fp64, SJ.plan);
     const size_t nsched = SJ.plan.sched.size(), nstream = SJ.plan.streamed.size();
     const size_t nps = nstream ? np : 0;
+    /* refused before anything is enqueued: an on-chip launch that is left
+     * behind would still use the workspace when the next call takes it */
+    if (nstream > kMaxStreamTiles)
+        return fail(CUPHU_ERR_INVALID, "at most 1024 streamed tiles per job");
 
     /* device layout */
     size_t post_bytes = 0;

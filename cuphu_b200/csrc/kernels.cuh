@@ -136,6 +136,7 @@ int upload_host_phase(const float *c64, const float *re, const float *im, size_t
 void compute_host_phase(const float *c64, const float *re, const float *im, size_t n, float *out);
 
 /* laplace.cu */
+constexpr int kMaxStreamTiles = 1024;   /* tiles of one launch_solve */
 int launch_solve(bool fp64, const TileDesc *tiles, int nitems, int ntiles, const SolverPlanes &P,
                  int plane_pitch, int plane_rows, TileState *st, double *part, SolverCtl *ctl,
                  const SolveParams &sp, int device, cudaStream_t s);

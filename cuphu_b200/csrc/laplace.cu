@@ -811,11 +811,10 @@ __device__ void phase_fold(const TileDesc &T, int li, const SolverPlanes &P, con
  * reduced redundantly (and identically) by every block whose slice touches
  * the tile; the block whose slice holds the tile's first item is its owner
  * for the global active-tile count. */
-constexpr int kMaxTiles = 1024;
 constexpr int kCacheTiles = 16;
 
 struct SliceCtl {
-    int pre[kMaxTiles + 1];          /* exclusive prefix of counted item numbers */
+    int pre[kMaxStreamTiles + 1];    /* exclusive prefix of counted item numbers */
     int s0, s1, t0, t1;              /* my slice in counted order, tiles it spans */
     int ncached;
     TileDesc d[kCacheTiles];
@@ -1653,7 +1652,7 @@ static int launch_solve_kernel(const TileDesc *tiles, int nitems, int ntiles,
                           SolverCtl *ctl, const SolveParams &sp, long long timeout_ns, int device,
                           cudaStream_t s)
 {
-    if (ntiles > kMaxTiles)
+    if (ntiles > kMaxStreamTiles)
         return fail(CUPHU_ERR_INVALID, "at most 1024 tiles per solver launch");
     /* the shape from the autotuner (job size = item count) */
     tune_note_items(nitems);

@@ -201,7 +201,8 @@ int cuphu_unwrap_device(const float *igram_c64, const float *phase_in, const flo
  * the split of an on-chip tile over the GPU, and with it the order in which
  * its FP64 dot products are summed, depends on the job: the sums agree to
  * about 1e-14, so that results are equal as a rule, but a last bit of the
- * solution, and at a pixel near a half cycle its cycle, may differ. */
+ * solution, and at a pixel near a half cycle its cycle, may differ.  At most
+ * 1024 tiles of a job may be streamed. */
 typedef struct CuPhuScene {
     const float         *igram_c64;   /* device, or NULL with phase      */
     const float         *phase;       /* device wrapped phase, or NULL   */

@@ -169,3 +169,33 @@ def test_skipped_barrier_of_a_streamed_job(torch_cuda, inputs, precision, which)
     check(rc)
     assert lib().cuphu_last_status(0) == 0
     assert all(same(a, b) for a, b in zip(got, want))
+
+
+def test_jobs_of_more_than_1024_tiles(torch_cuda, inputs):
+    """Refused where more than 1024 tiles are streamed, before any work is enqueued, and accepted
+    otherwise; the next call is not disturbed."""
+    t = torch_cuda
+    g = t.Generator(device="cuda")
+    g.manual_seed(8)
+
+    def data(nr, nc):
+        return (t.rand((nr, nc), generator=g, device="cuda") * 6.28,
+                t.rand((nr, nc), generator=g, device="cuda") * 0.5 + 0.4)
+
+    long, short = data(16401, 1), data(20, 30)
+    assert streamed([long[0].shape, short[0].shape], 1) == [1, 0]
+    scenes = (CuPhuScene * 1027)()
+    out = [(empty(d[0].shape, t.float32), empty(d[0].shape, t.int32)) for d in (long, short)]
+    for j in range(1027):
+        k = 0 if j < 1025 else 1
+        ph, c = (long, short)[k]
+        scenes[j] = CuPhuScene(None, ph.data_ptr(), c.data_ptr(), None, None, *ph.shape, 1, 1, 0, 0,
+                               5.0, out[k][0].data_ptr(), out[k][1].data_ptr())
+    p, o = default_params(), default_solve_options(precision=1, n_irls=0)
+    assert lib().cuphu_unwrap_batch_device(scenes, 1027, 0, C.byref(p), C.byref(o), None, None) == -2
+    rc, (want,), _ = solve(t, [short], 1)
+    check(rc)
+    rc, got, st = solve(t, [short] * 1100, 1)
+    check(rc)
+    assert st.ntiles == 1100
+    assert all(same(u, want) for u in got)
